@@ -196,7 +196,9 @@ def prepare(case, seed):
         cfg = get_lan_kde_config(case["model"])
         cfg["simulator"]["n_samples"] = case["samples"]
         st["pipe"] = BatchedKdePipeline(cfg, model_config[case["model"]], batch_size=case["sets"])
-        st["theta"] = st["pipe"].sampler.sample(n_samples=case["sets"], rng=rng)
+        # not the pipeline's own sampler: its parameter order, and with it the
+        # draws for one seed, differ between processes
+        st["theta"] = _theta(case["model"], case["sets"], rng)
     elif kind == "kde":
         st["rts"], st["choices"], st["soff"], st["qoff"], st["q"] = _kde_inputs(case, seed)
     elif kind == "surrogate":
