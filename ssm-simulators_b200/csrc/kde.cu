@@ -19,6 +19,8 @@
 // (group, query tile, point tile) is cut into equal contiguous ranges, one per
 // CTA of a persistent grid; query tiles cut between CTAs are finished by a
 // fix-up kernel that adds the CTAs' partial sums in CTA order.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "common.cuh"
@@ -52,24 +54,116 @@ __device__ __forceinline__ int choice_index(int32_t ch, const int32_t *cvals, in
     return -1;
 }
 
-__global__ void k_kde_count(const KdeFit a) {
-    const int64_t s = blockIdx.x;
-    __shared__ unsigned long long c_all[KDE_MAX_CHOICES], c_val[KDE_MAX_CHOICES];
-    if (threadIdx.x < KDE_MAX_CHOICES) c_all[threadIdx.x] = c_val[threadIdx.x] = 0ull;
+// The choice values in registers; NC is the compiled capacity (2, 4 or 16),
+// nc the number in use.
+template <int NC> struct ChoiceSet {
+    int32_t v[NC];
+    int nc;
+    __device__ __forceinline__ ChoiceSet(const int32_t *cvals, int n) : nc(n) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) v[c] = (c < n) ? __ldg(cvals + c) : 0;
+    }
+    __device__ __forceinline__ int index(int32_t ch) const {  // first match, -1: none
+        int ci = -1;
+#pragma unroll
+        for (int c = NC - 1; c >= 0; --c)
+            if (c < nc && v[c] == ch) ci = c;
+        return ci;
+    }
+};
+
+// The fit and the summary give every set a cluster of J CTAs (J = gridDim.x /
+// n_sets), each taking one contiguous slice of the set's samples: a handful of
+// sets still fills the GPU, and the slices' counts meet over distributed shared
+// memory instead of in a workspace.
+struct Slice {
+    int64_t set, lo, hi;
+    unsigned rank, J;
+};
+__device__ __forceinline__ Slice set_slice(const int64_t *soff, int64_t n_sets) {
+    Slice s;
+    s.J = (unsigned)(gridDim.x / n_sets);
+    s.set = blockIdx.x / s.J;
+    s.rank = (unsigned)(blockIdx.x - s.set * s.J);
+    const int64_t a = soff[s.set], n = soff[s.set + 1] - a;
+    s.lo = a + n * s.rank / s.J;
+    s.hi = a + n * (s.rank + 1) / s.J;
+    return s;
+}
+
+// f(rt, choice) for the samples [lo, hi) in no particular order: 16-byte loads
+// where both arrays allow them (same offset from a 16-byte boundary), scalar
+// loads at the ragged ends and otherwise.
+template <class F>
+__device__ __forceinline__ void for_each_sample(const float *rts, const int32_t *choices, int64_t lo, int64_t hi,
+                                                F f) {
+    const bool vec = ((((uintptr_t)rts ^ (uintptr_t)choices) & 15u) == 0);
+    int64_t v0 = hi, v1 = hi;
+    if (vec) {
+        v0 = min(hi, lo + (int64_t)((4 - (((uintptr_t)(rts + lo) >> 2) & 3)) & 3));
+        v1 = v0 + ((hi - v0) & ~(int64_t)3);
+    }
+    for (int64_t i = lo + threadIdx.x; i < v0; i += blockDim.x) f(rts[i], choices[i]);
+#pragma unroll 4
+    for (int64_t i = v0 + 4 * (int64_t)threadIdx.x; i < v1; i += 4 * (int64_t)blockDim.x) {
+        const float4 r = *reinterpret_cast<const float4 *>(rts + i);
+        const int4 c = *reinterpret_cast<const int4 *>(choices + i);
+        f(r.x, c.x);
+        f(r.y, c.y);
+        f(r.z, c.z);
+        f(r.w, c.w);
+    }
+    for (int64_t i = v1 + threadIdx.x; i < hi; i += blockDim.x) f(rts[i], choices[i]);
+}
+
+// Samples per choice, with and without omissions.  Bound by reading 8 bytes a
+// sample: the counts stay in registers (one compare-and-add per choice), are
+// summed over the warp by one reduction each, and the cluster's CTAs meet in
+// rank 0.  Two 64-bit shared counters per choice, which every lane hit, had
+// serialised the whole pass: 128 sets of 20 000 samples 831 us, 256 of 50 000
+// 2 500 us.
+template <int NC>
+__global__ void __launch_bounds__(256) k_kde_count(const KdeFit a) {
+    namespace cg = cooperative_groups;
+    __shared__ unsigned int tot[2 * NC];
+    const Slice sl = set_slice(a.soff, a.n_sets);
+    const ChoiceSet<NC> cs(a.cvals, a.nc);
+    if (threadIdx.x < 2 * NC) tot[threadIdx.x] = 0u;
     __syncthreads();
-    const int64_t lo = a.soff[s], hi = a.soff[s + 1];
-    for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-        const int ci = choice_index(a.choices[i], a.cvals, a.nc);
-        if (ci >= 0) {
-            atomicAdd(&c_all[ci], 1ull);
-            if (a.rts[i] != -999.f) atomicAdd(&c_val[ci], 1ull);
+    unsigned int all[NC], val[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) all[c] = val[c] = 0u;
+    for_each_sample(a.rts, a.choices, sl.lo, sl.hi, [&](float rt, int32_t ch) {
+        const int ci = cs.index(ch);
+        const bool kept = (rt != -999.f);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            all[c] += (ci == c);
+            val[c] += (ci == c && kept);
+        }
+    });
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const unsigned int x = __reduce_add_sync(0xffffffffu, all[c]), y = __reduce_add_sync(0xffffffffu, val[c]);
+        if (lane == 0) {
+            atomicAdd(&tot[c], x);
+            atomicAdd(&tot[NC + c], y);
         }
     }
-    __syncthreads();
-    if (threadIdx.x < a.nc) {
-        a.count_all[s * a.nc + threadIdx.x] = (int64_t)c_all[threadIdx.x];
-        a.n_valid[s * a.nc + threadIdx.x] = (int64_t)c_val[threadIdx.x];
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();
+    if (sl.rank == 0 && threadIdx.x < a.nc) {
+        int64_t x = 0, y = 0;
+        for (unsigned j = 0; j < sl.J; ++j) {
+            const unsigned int *t = cl.map_shared_rank(tot, j);
+            x += t[threadIdx.x];
+            y += t[NC + threadIdx.x];
+        }
+        a.count_all[sl.set * a.nc + threadIdx.x] = x;
+        a.n_valid[sl.set * a.nc + threadIdx.x] = y;
     }
+    cl.sync();  // the slices' shared counters stay until rank 0 has read them
 }
 
 // Exclusive prefix sum of n int64 values into out[0..n] (one CTA of 1024).
@@ -107,54 +201,6 @@ __global__ void k_scan_i64(const int64_t *in, int64_t n, int64_t *out) {
     if (threadIdx.x == 0) out[n] = carry;
 }
 
-// Stable per-choice compaction of log(rt - shift) into the group regions.
-__global__ void __launch_bounds__(256) k_kde_scatter(const KdeFit a) {
-    const int64_t s = blockIdx.x;
-    constexpr int W = 8;
-    __shared__ int64_t base[KDE_MAX_CHOICES];
-    __shared__ int wcnt[W][KDE_MAX_CHOICES];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned lt = (1u << lane) - 1u;
-    if (threadIdx.x < a.nc) base[threadIdx.x] = a.poff[s * a.nc + threadIdx.x];
-    const double sh = a.shift ? a.shift[s] : 0.0;
-    __syncthreads();
-    const int64_t lo = a.soff[s], hi = a.soff[s + 1];
-    for (int64_t c0 = lo; c0 < hi; c0 += blockDim.x) {
-        const int64_t i = c0 + threadIdx.x;
-        int ci = -1;
-        float rt = 0.f;
-        if (i < hi) {
-            rt = a.rts[i];
-            if (rt != -999.f) ci = choice_index(a.choices[i], a.cvals, a.nc);
-        }
-        int rank = 0;
-        for (int c = 0; c < a.nc; ++c) {
-            const unsigned m = __ballot_sync(0xffffffffu, ci == c);
-            if (ci == c) rank = __popc(m & lt);
-            if (lane == 0) wcnt[warp][c] = __popc(m);
-        }
-        __syncthreads();
-        if (ci >= 0) {
-            int64_t pos = base[ci] + rank;
-            for (int w = 0; w < warp; ++w) pos += wcnt[w][ci];
-            // kernels sit on float32 log of the float32 (displaced) rt; with a
-            // shift the rt is displaced in float64 and stored as float32, and the
-            // bandwidth uses log(exp(float32 log rt) - shift) in float64
-            // (kde_class.py:174-186, 478-493)
-            const float r = a.shift ? __double2float_rn((double)rt - sh) : rt;
-            a.points[pos] = __double2float_rn(log((double)r));
-            if (a.bwvals) a.bwvals[pos] = log(exp((double)__double2float_rn(log((double)rt))) - sh);
-        }
-        __syncthreads();
-        if (threadIdx.x < a.nc) {
-            int64_t t = 0;
-            for (int w = 0; w < W; ++w) t += wcnt[w][threadIdx.x];
-            base[threadIdx.x] += t;
-        }
-        __syncthreads();
-    }
-}
-
 __device__ __forceinline__ double block_sum_f64(double v, double *red) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -171,24 +217,184 @@ __device__ __forceinline__ double block_sum_f64(double v, double *red) {
     return r;
 }
 
-// Silverman bandwidth (kde_class.py:508-553) and normaliser per group.
-__global__ void __launch_bounds__(256) k_kde_stats(const KdeFit a) {
-    const int64_t g = blockIdx.x;
-    const int64_t s = g / a.nc;
-    __shared__ double red[32];
-    const int64_t lo = a.poff[g], n = a.poff[g + 1] - lo;
-    double sum = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x)
-        sum += a.bwvals ? a.bwvals[lo + i] : (double)a.points[lo + i];
-    const double mean = block_sum_f64(sum, red) / (double)(n > 0 ? n : 1);
-    double ss = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const double d = (a.bwvals ? a.bwvals[lo + i] : (double)a.points[lo + i]) - mean;
-        ss += d * d;
+// Stable per-choice compaction of log(rt - shift) into the group regions, then
+// Silverman's bandwidth (kde_class.py:508-553) and the normaliser of each group.
+//
+// Each CTA of the set's cluster first counts its own slice (the samples are in
+// L2 after k_kde_count), so its first position per choice follows from the
+// lower ranks' counts; then it walks the slice in chunks of 1 024 samples, four
+// consecutive ones per thread.  Ranks inside a chunk come from a warp scan of
+// byte-packed counts (four choices in one word, at most 128 each) and the warps'
+// totals, one barrier per chunk.  Sums of the log-rts are taken on the way;
+// the squared deviations from the mean are a second pass over the group's
+// points, still in L2, shared by the cluster.  What remains is the float64
+// logarithm of every sample.  One CTA per set with a barrier pair per 256 samples
+// and the moments in a kernel of their own had taken 87 + 13 us for 128 sets of
+// 20 000 samples and 348 + 45 us for 256 of 50 000.
+template <int NC>
+__global__ void __launch_bounds__(256) k_kde_scatter(const KdeFit a) {
+    namespace cg = cooperative_groups;
+    constexpr int W = 8, NW = (NC + 3) / 4;
+    __shared__ unsigned int tot[NC];
+    __shared__ __align__(16) unsigned int wtot[2][NW][W];
+    __shared__ double red[32], csum[NC], css[NC];
+    cg::cluster_group cl = cg::this_cluster();
+    const Slice sl = set_slice(a.soff, a.n_sets);
+    const ChoiceSet<NC> cs(a.cvals, a.nc);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double sh = a.shift ? a.shift[sl.set] : 0.0;
+
+    // this slice's counts, then the position of its first sample of each choice
+    int64_t base[NC];
+    {
+        if (threadIdx.x < NC) tot[threadIdx.x] = 0u;
+        __syncthreads();
+        if (sl.J > 1) {
+            unsigned int val[NC];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) val[c] = 0u;
+            for_each_sample(a.rts, a.choices, sl.lo, sl.hi, [&](float rt, int32_t ch) {
+                const int ci = (rt != -999.f) ? cs.index(ch) : -1;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) val[c] += (ci == c);
+            });
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const unsigned int y = __reduce_add_sync(0xffffffffu, val[c]);
+                if (lane == 0) atomicAdd(&tot[c], y);
+            }
+        }
+        cl.sync();
+#pragma unroll
+        for (int c = 0; c < NC; ++c) base[c] = (c < a.nc) ? a.poff[sl.set * a.nc + c] : 0;
+        for (unsigned j = 0; j < sl.rank; ++j) {
+            const unsigned int *t = cl.map_shared_rank(tot, j);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) base[c] += t[c];
+        }
     }
-    const double var = block_sum_f64(ss, red) / (double)(n > 0 ? n : 1);
-    if (threadIdx.x == 0) {
-        const int64_t N = a.soff[s + 1] - a.soff[s];
+    double s1[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) s1[c] = 0.0;
+
+    const bool vec = ((((uintptr_t)a.rts ^ (uintptr_t)a.choices) & 15u) == 0);
+    const int64_t start = sl.lo - (int64_t)(((uintptr_t)(a.rts + sl.lo) >> 2) & 3);  // 16-byte boundary at or before lo
+    int buf = 0;
+    for (int64_t c0 = start; c0 < sl.hi; c0 += 1024, buf ^= 1) {
+        const int64_t i0 = c0 + 4 * threadIdx.x;
+        float rt[4];
+        int ci[4];
+        if (vec && i0 >= sl.lo && i0 + 4 <= sl.hi) {
+            const float4 r = *reinterpret_cast<const float4 *>(a.rts + i0);
+            const int4 h = *reinterpret_cast<const int4 *>(a.choices + i0);
+            rt[0] = r.x; rt[1] = r.y; rt[2] = r.z; rt[3] = r.w;
+            ci[0] = cs.index(h.x); ci[1] = cs.index(h.y); ci[2] = cs.index(h.z); ci[3] = cs.index(h.w);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const bool in = (i0 + q >= sl.lo) && (i0 + q < sl.hi);
+                rt[q] = in ? a.rts[i0 + q] : -999.f;
+                ci[q] = in ? cs.index(a.choices[i0 + q]) : -1;
+            }
+        }
+        unsigned int own[NW], inc[NW];
+#pragma unroll
+        for (int w = 0; w < NW; ++w) own[w] = 0u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (rt[q] == -999.f) ci[q] = -1;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) own[c / 4] += (ci[q] == c) ? (1u << (8 * (c % 4))) : 0u;
+        }
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            inc[w] = own[w];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned int y = __shfl_up_sync(0xffffffffu, inc[w], o);
+                if (lane >= o) inc[w] += y;
+            }
+            if (lane == 31) wtot[buf][w][warp] = inc[w];
+        }
+        __syncthreads();  // the other buffer's readers are past it once everybody is here
+        int64_t pos[NC];
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            // the eight warps' totals as 16-bit fields: choices 4w, 4w+2 and 4w+1, 4w+3
+            unsigned int pe = 0, po = 0, te = 0, to = 0;
+#pragma unroll
+            for (int k = 0; k < W; ++k) {
+                const unsigned int x = wtot[buf][w][k], e = x & 0x00ff00ffu, o = (x >> 8) & 0x00ff00ffu;
+                te += e;
+                to += o;
+                pe += (k < warp) ? e : 0u;
+                po += (k < warp) ? o : 0u;
+            }
+            const unsigned int ex = inc[w] - own[w];
+            pe += ex & 0x00ff00ffu;
+            po += (ex >> 8) & 0x00ff00ffu;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int c = 4 * w + q;
+                if (c < NC) {
+                    pos[c] = base[c] + (((q & 1) ? po : pe) >> (16 * (q / 2)) & 0xffffu);
+                    base[c] += ((q & 1) ? to : te) >> (16 * (q / 2)) & 0xffffu;
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (ci[q] < 0) continue;
+            int64_t at = 0;
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                if (ci[q] == c) at = pos[c]++;
+            // kernels sit on float32 log of the float32 (displaced) rt; with a
+            // shift the rt is displaced in float64 and stored as float32, and the
+            // bandwidth uses log(exp(float32 log rt) - shift) in float64
+            // (kde_class.py:174-186, 478-493)
+            const float r = a.shift ? __double2float_rn((double)rt[q] - sh) : rt[q];
+            const float x = __double2float_rn(log((double)r));
+            a.points[at] = x;
+            double m = (double)x;
+            if (a.bwvals) {
+                m = log(exp((double)__double2float_rn(log((double)rt[q]))) - sh);
+                a.bwvals[at] = m;
+            }
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                if (ci[q] == c) s1[c] += m;
+        }
+    }
+    // mean of each group: the ranks' sums in rank order
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+        if (c < a.nc) {
+            const double t = block_sum_f64(s1[c], red);
+            if (threadIdx.x == 0) csum[c] = t;
+        }
+    cl.sync();  // also orders the cluster's point writes before the reads below
+    for (int c = 0; c < a.nc; ++c) {
+        const int64_t g = sl.set * a.nc + c, lo = a.poff[g], n = a.poff[g + 1] - lo;
+        double mean = 0.0;
+        for (unsigned j = 0; j < sl.J; ++j) mean += cl.map_shared_rank(csum, j)[c];
+        mean /= (double)(n > 0 ? n : 1);
+        double ss = 0.0;
+        for (int64_t i = (int64_t)sl.rank * blockDim.x + threadIdx.x; i < n; i += (int64_t)sl.J * blockDim.x) {
+            const double d = (a.bwvals ? __ldcg(a.bwvals + lo + i) : (double)__ldcg(a.points + lo + i)) - mean;
+            ss += d * d;
+        }
+        const double t = block_sum_f64(ss, red);
+        if (threadIdx.x == 0) css[c] = t;
+    }
+    cl.sync();
+    if (sl.rank == 0 && threadIdx.x < a.nc) {
+        const int c = threadIdx.x;
+        const int64_t g = sl.set * a.nc + c, n = a.poff[g + 1] - a.poff[g];
+        const int64_t N = a.soff[sl.set + 1] - a.soff[sl.set];
+        double ss = 0.0;
+        for (unsigned j = 0; j < sl.J; ++j) ss += cl.map_shared_rank(css, j)[c];
+        const double var = ss / (double)(n > 0 ? n : 1);
         const double p = (N > 0) ? (double)a.count_all[g] / (double)N : 0.0;
         a.prop[g] = p;
         if (n == 0) {
@@ -202,6 +408,7 @@ __global__ void __launch_bounds__(256) k_kde_stats(const KdeFit a) {
             a.lognorm[g] = log(p) - log((double)n) - log(h) - 0.5 * KDE_LOG_2PI;
         }
     }
+    cl.sync();  // rank 0 has read the others' sums
 }
 
 struct KdeEval {
@@ -595,6 +802,41 @@ __global__ void __launch_bounds__(256) k_set_summary(const SetSummary a) {
     }
 }
 
+// CTAs per set of the per-set kernels (a cluster, at most the portable 8): the
+// fewest that give every SM four 256-thread CTAs.
+static unsigned ctas_per_set(int64_t n_sets) {
+    unsigned J = 1;
+    while (J < 8 && n_sets * J < (int64_t)sm_count() * 4) J *= 2;
+    return J;
+}
+
+template <class K, class A>
+static int launch_per_set(K kernel, const A &args, int64_t n_sets, size_t smem, cudaStream_t st) {
+    const unsigned J = ctas_per_set(n_sets);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n_sets * J));
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = J;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    SSM_CUDA(cudaLaunchKernelEx(&cfg, kernel, args));
+    return SSM_OK;
+}
+
+template <int NC>
+static int kde_fit(const KdeFit &a, cudaStream_t st) {
+    int rc = launch_per_set(k_kde_count<NC>, a, a.n_sets, 0, st);
+    if (rc != SSM_OK) return rc;
+    k_scan_i64<<<1, 1024, 0, st>>>(a.n_valid, a.n_sets * a.nc, a.poff);
+    SSM_CUDA(cudaGetLastError());
+    return launch_per_set(k_kde_scatter<NC>, a, a.n_sets, 0, st);
+}
+
 }  // namespace ssm
 
 extern "C" {
@@ -638,16 +880,10 @@ int ssm_kde_fit(const float *rts, const int32_t *choices, int64_t n_sets,
     KdeFit a{rts, choices, n_sets, sample_offsets, choice_values, n_choices, displace,
              displace ? displaced_logs : nullptr, count_all, n_valid, point_offsets, points,
              bandwidth, log_norm, proportion};
-    const int64_t G = n_sets * n_choices;
-    k_kde_count<<<(unsigned)n_sets, 256, 0, st>>>(a);
-    SSM_CUDA(cudaGetLastError());
-    k_scan_i64<<<1, 1024, 0, st>>>(n_valid, G, point_offsets);
-    SSM_CUDA(cudaGetLastError());
-    k_kde_scatter<<<(unsigned)n_sets, 256, 0, st>>>(a);
-    SSM_CUDA(cudaGetLastError());
-    k_kde_stats<<<(unsigned)G, 256, 0, st>>>(a);
-    SSM_CUDA(cudaGetLastError());
-    return SSM_OK;
+    SSM_REQUIRE(n_sets < (int64_t)1 << 28, "too many sets for one launch");
+    if (n_choices <= 2) return kde_fit<2>(a, st);
+    if (n_choices <= 4) return kde_fit<4>(a, st);
+    return kde_fit<KDE_MAX_CHOICES>(a, st);
 }
 
 }  // extern "C"
