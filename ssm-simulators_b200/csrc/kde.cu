@@ -10,18 +10,17 @@
 // Evaluation.  For a query log-rt q of group g the reference evaluates
 //   log p_c + log( 1/(n h sqrt(2 pi)) sum_j exp(-(q - x_j)^2 / (2 h^2)) ) - q
 // exactly (scikit-learn with atol = rtol = 0).  k_kde_eval tiles the group's
-// points through shared memory, keeps QPT queries per thread in registers
+// points through shared memory, keeps up to four queries per lane in registers
 // (q split into float hi + lo parts so q - x_j keeps full precision), evaluates
 // each kernel term as ex2(-(d s)^2) on the SFU and sums in float over 32 terms
 // before adding into a float64 accumulator.  Groups differ in cost by orders
 // of magnitude (queries x points), so the work is scheduled Stream-K style
-// (Osama, Merrill, Cecka, Garland & Owens, PPoPP'23): the iteration space
-// (group, query tile, point tile) is cut into equal contiguous ranges, one per
-// CTA of a persistent grid; query tiles cut between CTAs are finished by a
-// fix-up kernel that adds the CTAs' partial sums in CTA order.
+// (Osama, Merrill, Cecka, Garland & Owens, PPoPP'23): the cost space (group,
+// unit of up to 16 rows of 32 queries, point tile) is cut into equal contiguous
+// ranges, one per CTA of a persistent grid; units cut between CTAs are finished
+// by a fix-up kernel that adds the CTAs' partial sums in CTA order.
 #include <cooperative_groups.h>
 
-#include <algorithm>
 
 #include "common.cuh"
 
@@ -423,21 +422,24 @@ struct KdeEval {
     const int64_t *soff;
     const double *shift;
     double lb, eps, max_t;
-    // Stream-K schedule (see ssm_kde_eval): units are (group, tile of KDE_QT
-    // queries); a unit's iterations are its group's point tiles.
-    int64_t *uoff;     // [G + 1] first unit of each group
-    int64_t *ucnt;     // [G] units per group (scan input)
-    int64_t *ioff;     // [u_max + 1] first iteration of each unit
-    int64_t *icnt;     // [u_max] iterations per unit (scan input)
+    // Stream-K schedule (see k_kde_plan): units are (group, up to KDE_ROWS rows
+    // of 32 queries); unit u's cost span is [ioff[u], ioff[u + 1]).
+    int64_t *head;     // [3] number of units, total cost, CTAs that share it
+    int64_t *ioff;     // [u_max + 1]
+    int32_t *ugroup;   // [u_max] the unit's group
+    int32_t *uidx;     // [u_max] its place among the group's units
+    int32_t *tail;     // [P] unit whose first part CTA c holds (-1: none)
+    int32_t *link;     // [P] what CTA c holds of the unit begun before it (SPLIT_*)
     int64_t u_max;     // capacity of the unit arrays
     double *slots;     // [P][2][KDE_QT] partial sums of units split between CTAs
     int64_t P;         // CTAs of the evaluation grid
 };
 
-constexpr int KDE_TILE = 2048;
-constexpr int KDE_QPT = 4;
+constexpr int KDE_TILE = 512;     // points staged in shared memory at a time (a multiple of 32)
 constexpr int KDE_THREADS = 128;
-constexpr int KDE_QT = KDE_QPT * KDE_THREADS;
+constexpr int KDE_ROWS = 16;      // rows of 32 queries per unit, four per warp at most
+constexpr int KDE_QT = 32 * KDE_ROWS;
+enum { SPLIT_PART = 1, SPLIT_LAST = 2, SPLIT_NONE = 3 };
 
 __device__ __forceinline__ int64_t upper_index(const int64_t *off, int64_t n, int64_t x) {
     // largest i in [0, n) with off[i] <= x (off non-decreasing, off[0] <= x)
@@ -449,38 +451,96 @@ __device__ __forceinline__ int64_t upper_index(const int64_t *off, int64_t n, in
     return lo;
 }
 
-__global__ void k_kde_units(const KdeEval a) {
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < a.G; g += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t m = a.qoff[g + 1] - a.qoff[g];
-        a.ucnt[g] = (m + KDE_QT - 1) / KDE_QT;
-    }
+// Rows of 32 queries [r0, r1) of unit k of a group with m queries: the
+// group's ceil(m / 32) rows spread evenly over its ceil(m / KDE_QT) units.
+struct UnitRows {
+    int64_t r0, r1;
+};
+__device__ __forceinline__ int64_t group_units(int64_t m) { return m > 0 ? (m + KDE_QT - 1) / KDE_QT : 0; }
+__device__ __forceinline__ UnitRows unit_rows(int64_t m, int64_t k) {
+    const int64_t rows = (m + 31) / 32, T = group_units(m);
+    return {rows * k / T, rows * (k + 1) / T};
 }
+__device__ __forceinline__ int64_t point_tiles(int64_t n) { return n > 0 ? (n + KDE_TILE - 1) / KDE_TILE : 1; }
 
-__global__ void k_kde_unit_iters(const KdeEval a) {
-    const int64_t U = min(a.uoff[a.G], a.u_max);
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < a.u_max; u += (int64_t)gridDim.x * blockDim.x) {
-        int64_t it = 0;
-        if (u < U) {
-            const int64_t g = upper_index(a.uoff, a.G + 1, u);
-            const int64_t n = a.poff[g + 1] - a.poff[g];
-            it = (n > 0) ? (n + KDE_TILE - 1) / KDE_TILE : 1;
+// The Stream-K schedule, by one CTA: a unit of R rows costs R + 1 per point
+// tile (the 1 for staging the tile), a group's units R_group + T in all, so one
+// two-value scan over the groups places every unit.
+__global__ void __launch_bounds__(1024) k_kde_plan(const KdeEval a) {
+    __shared__ int64_t wu[32], wi[32];
+    __shared__ int64_t wt[32];
+    int64_t n_tiles = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t cu = 0, ci = 0;  // units and cost of the groups before this pass
+    for (int64_t b = 0; b < a.G; b += blockDim.x) {
+        const int64_t g = b + threadIdx.x;
+        int64_t m = 0, T = 0, tiles = 0, cost = 0;
+        if (g < a.G) {
+            m = a.qoff[g + 1] - a.qoff[g];
+            T = group_units(m);
+            tiles = point_tiles(a.poff[g + 1] - a.poff[g]);
+            cost = (m > 0) ? tiles * ((m + 31) / 32 + T) : 0;
+            n_tiles += tiles * T;
         }
-        a.icnt[u] = it;
+        int64_t x = T, y = cost;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t p = __shfl_up_sync(0xffffffffu, x, o), q = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= o) {
+                x += p;
+                y += q;
+            }
+        }
+        __syncthreads();
+        if (lane == 31) {
+            wu[warp] = x;
+            wi[warp] = y;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            int64_t p = wu[lane], q = wi[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const int64_t pp = __shfl_up_sync(0xffffffffu, p, o), qq = __shfl_up_sync(0xffffffffu, q, o);
+                if (lane >= o) {
+                    p += pp;
+                    q += qq;
+                }
+            }
+            wu[lane] = p;
+            wi[lane] = q;
+        }
+        __syncthreads();
+        int64_t u = cu + (warp > 0 ? wu[warp - 1] : 0) + x - T;
+        int64_t i = ci + (warp > 0 ? wi[warp - 1] : 0) + y - cost;
+        for (int64_t k = 0; k < T && u < a.u_max; ++k, ++u) {
+            const UnitRows r = unit_rows(m, k);
+            a.ioff[u] = i;
+            a.ugroup[u] = (int32_t)g;
+            a.uidx[u] = (int32_t)k;
+            i += tiles * (r.r1 - r.r0 + 1);
+        }
+        cu += wu[31];
+        ci += wi[31];
+    }
+    for (int o = 16; o > 0; o >>= 1) n_tiles += __shfl_down_sync(0xffffffffu, n_tiles, o);
+    if (lane == 0) wt[warp] = n_tiles;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        a.head[0] = min(cu, a.u_max);
+        a.head[1] = ci;
+        // no more CTAs than tiles: a unit cut between CTAs without a tile each
+        // would only make the fix-up's chain longer (one set of
+        // 20 000 points, 1 000 queries: fix-up 108 -> 12 us)
+        n_tiles = 0;
+        for (int w = 0; w < 32; ++w) n_tiles += wt[w];
+        a.head[2] = min(a.P, n_tiles);
+        a.ioff[min(cu, a.u_max)] = ci;
     }
 }
 
-// first iteration of CTA c: floor(c * I / P) (c <= P < 2^16 and I < 2^46, so
+// first cost index of CTA c: floor(c * I / P) (c <= P < 2^16 and I < 2^46, so
 // the product fits in 64 bits)
 __device__ __forceinline__ int64_t sk_begin(int64_t c, int64_t I, int64_t P) {
     return (c * I) / P;
-}
-// the CTA whose iteration range holds iteration i (empty CTAs own nothing)
-__device__ __forceinline__ int64_t sk_owner(int64_t i, int64_t I, int64_t P) {
-    int64_t c = (i * P) / I;
-    if (c > P - 1) c = P - 1;
-    while (c > 0 && sk_begin(c, I, P) > i) --c;
-    while (c + 1 < P && sk_begin(c + 1, I, P) <= i) ++c;
-    return c;
 }
 
 // log-likelihood of one query from its kernel sum acc (kde_class.py:188-329)
@@ -500,119 +560,189 @@ __device__ __forceinline__ double kde_finalize(const KdeEval &a, int64_t g, int6
     return ll;
 }
 
-// Each thread holds KDE_QPT queries of the unit (q split into float hi + lo
-// parts so q - x_j keeps full precision), the group's points stream through
-// shared memory one tile per iteration, and each kernel term is
-// ex2(-(d s)^2) on the SFU, summed in float over 32 terms before it is added
-// into a float64 accumulator.
-__global__ void __launch_bounds__(KDE_THREADS, 7) k_kde_eval(const KdeEval a) {
-    __shared__ __align__(16) float tile[KDE_TILE];
-    const int64_t U = min(a.uoff[a.G], a.u_max);
-    const int64_t I = a.ioff[a.u_max];
-    const int64_t c = blockIdx.x;
-    const int64_t i0 = sk_begin(c, I, a.P), i1 = sk_begin(c + 1, I, a.P);
-    if (i0 >= i1) return;
-    int64_t u = upper_index(a.ioff, U, i0);
-    int64_t g = upper_index(a.uoff, a.G + 1, u);
-    for (int64_t it = i0; it < i1;) {
-        while (a.uoff[g + 1] <= u) ++g;
-        const int64_t ubeg = a.ioff[u], uend = a.ioff[u + 1];
-        const int64_t lo = it, hi = (uend < i1) ? uend : i1;
-        const int64_t q0 = a.qoff[g] + (u - a.uoff[g]) * KDE_QT, q1 = a.qoff[g + 1];
-        const int64_t p0 = a.poff[g], n = a.poff[g + 1] - p0;
-        const double hg = a.h[g];
-        const double sh = a.shift ? a.shift[g / a.nc] : 0.0;
-        // 2^(-(d*sc)^2) = exp(-d^2 / (2 h^2))
-        const float sc = (n > 0) ? (float)(0.8493218002880191 / hg) : 0.f;  // sqrt(log2(e)/2) / h
-        float qhi[KDE_QPT], qlo[KDE_QPT], part[KDE_QPT];
-        double acc[KDE_QPT];
+// Packed pairs of float32 (two IEEE operations per instruction, the same
+// results as the scalar ones).
+__device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul_f2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float ex2_neg_sum(uint64_t e) {  // 2^-lo + 2^-hi
+    float lo, hi, r0, r1;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(e));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(-lo));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(-hi));
+    return r0 + r1;
+}
+
+// Kernel sums of NJ queries per lane over one staged tile of 32 * n32 points
+// (padding points weigh exactly 0): float over 32 terms, then float64.
+template <int NJ>
+__device__ __forceinline__ void kde_tile(const float *tile, int n32, const float *qhi, const float *qlo, float sc,
+                                         double *acc) {
+    const uint64_t minus1 = pack_f2(-1.f, -1.f), sc2 = pack_f2(sc, sc);
+    uint64_t h2[NJ], l2[NJ];
 #pragma unroll
-        for (int j = 0; j < KDE_QPT; ++j) {
-            const int64_t qi = q0 + threadIdx.x + (int64_t)j * KDE_THREADS;
-            const double lq = log(fmax((qi < q1) ? a.q_rt[qi] - sh : 1.0, a.eps));
-            qhi[j] = (float)lq;
-            qlo[j] = (float)(lq - (double)qhi[j]);
-            part[j] = 0.f;
-            acc[j] = 0.0;
-        }
-        for (int64_t t = lo - ubeg; t < hi - ubeg && n > 0; ++t) {
-            const int64_t b0 = t * KDE_TILE;
-            const int cnt = (int)min((int64_t)KDE_TILE, n - b0);
-            __syncthreads();
-            for (int i = threadIdx.x; i < KDE_TILE; i += KDE_THREADS)
-                tile[i] = (i < cnt) ? __ldg(a.points + p0 + b0 + i) : qhi[0] + 1e30f;  // padding: zero weight
-            __syncthreads();
-            const float4 *t4 = reinterpret_cast<const float4 *>(tile);
-            const int n4 = (cnt + 3) >> 2;
-            for (int k0 = 0; k0 < n4; k0 += 8) {
+    for (int j = 0; j < NJ; ++j) {
+        h2[j] = pack_f2(qhi[j], qhi[j]);
+        l2[j] = pack_f2(qlo[j], qlo[j]);
+    }
+    const ulonglong2 *t4 = reinterpret_cast<const ulonglong2 *>(tile);
+#pragma unroll 1
+    for (int k0 = 0; k0 < n32; ++k0) {
+        float part[NJ];
 #pragma unroll
-                for (int kk = 0; kk < 8; ++kk) {
-                    const float4 x = t4[min(k0 + kk, KDE_TILE / 4 - 1)];
-                    const bool live = (k0 + kk) < n4;
+        for (int j = 0; j < NJ; ++j) part[j] = 0.f;
 #pragma unroll
-                    for (int j = 0; j < KDE_QPT; ++j) {
-                        float d, e, r0, r1, r2, r3;
-                        d = ((qhi[j] - x.x) + qlo[j]) * sc; e = -d * d;
-                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(e));
-                        d = ((qhi[j] - x.y) + qlo[j]) * sc; e = -d * d;
-                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(e));
-                        d = ((qhi[j] - x.z) + qlo[j]) * sc; e = -d * d;
-                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r2) : "f"(e));
-                        d = ((qhi[j] - x.w) + qlo[j]) * sc; e = -d * d;
-                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r3) : "f"(e));
-                        if (live) part[j] += (r0 + r1) + (r2 + r3);
-                    }
-                }
+        for (int kk = 0; kk < 8; ++kk) {
+            const ulonglong2 x = t4[8 * k0 + kk];
 #pragma unroll
-                for (int j = 0; j < KDE_QPT; ++j) {
-                    acc[j] += (double)part[j];
-                    part[j] = 0.f;
-                }
+            for (int j = 0; j < NJ; ++j) {
+                const uint64_t a = mul_f2(add_f2(fma_f2(x.x, minus1, h2[j]), l2[j]), sc2);
+                const uint64_t b = mul_f2(add_f2(fma_f2(x.y, minus1, h2[j]), l2[j]), sc2);
+                part[j] += ex2_neg_sum(mul_f2(a, a)) + ex2_neg_sum(mul_f2(b, b));
             }
         }
-        if (lo == ubeg && hi == uend) {
 #pragma unroll
-            for (int j = 0; j < KDE_QPT; ++j) {
-                const int64_t qi = q0 + threadIdx.x + (int64_t)j * KDE_THREADS;
-                if (qi < q1) {
+        for (int j = 0; j < NJ; ++j) acc[j] += (double)part[j];
+    }
+}
+
+// Lanes hold queries (q split into float hi + lo parts so q - x_j keeps full
+// precision), the group's points stream through shared memory one tile at a
+// time, and each kernel term is ex2(-(d s)^2).  Bound by the SFU: one ex2 per
+// term, 16 a clock and SM.  A unit's rows of 32 queries go round the CTA's four
+// warps (up to four each, the first warp rotating with the unit), so a group
+// pays for its queries to a multiple of 32 instead of 512, and the rest of a
+// term -- subtract, add the low part, scale, square -- is packed two points to
+// an instruction: 4 issue slots a term against the SFU's 8 clocks a warp (6 and
+// the tail's selects before).  Measured, 256 groups of about 10 000 points
+// and 500 queries each: 763 -> 476 us (XU pipe 83 % of the active cycles); 512 of
+// 25 000 points and 450 queries: 3 530 -> 2 538 us.  7 CTAs per SM: 479 us, 6: 497,
+// 8: 509.  Tiles of 2 048, 1 024, 512 and 256 points: 530, 479, 472 and 468 us,
+// and on a single set of 20 000 points 49, 37, 22 and 20 us.
+__global__ void __launch_bounds__(KDE_THREADS, 7) k_kde_eval(const KdeEval a) {
+    __shared__ __align__(16) float tile[KDE_TILE];
+    const int64_t U = a.head[0], I = a.head[1], P = a.head[2];
+    const int64_t c = blockIdx.x;
+    const int64_t i0 = (c < P) ? sk_begin(c, I, P) : I, i1 = (c < P) ? sk_begin(c + 1, I, P) : I;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int tail = -1;
+    if (threadIdx.x == 0) a.link[c] = SPLIT_NONE;
+    if (i0 < i1) {
+        for (int64_t u = upper_index(a.ioff, U, i0); u < U; ++u) {
+            const int64_t ubeg = a.ioff[u], uend = a.ioff[u + 1];
+            if (ubeg >= i1) break;
+            const int64_t g = a.ugroup[u], qa = a.qoff[g], q1 = a.qoff[g + 1];
+            const UnitRows rows = unit_rows(q1 - qa, a.uidx[u]);
+            const int R = (int)(rows.r1 - rows.r0);
+            const int64_t p0 = a.poff[g], n = a.poff[g + 1] - p0, tiles = point_tiles(n);
+            // this CTA computes the tiles whose first cost index is in [i0, i1)
+            const int64_t t0 = (i0 > ubeg) ? (i0 - ubeg + R) / (R + 1) : 0;
+            const int64_t t1 = (i1 < uend) ? min((i1 - ubeg + R) / (R + 1), tiles) : tiles;
+            if (t0 >= tiles) continue;
+            if (t0 >= t1) continue;
+            if (i0 > ubeg && threadIdx.x == 0) a.link[c] = (t1 == tiles) ? SPLIT_LAST : SPLIT_PART;
+            const int64_t q0 = qa + 32 * rows.r0;
+            const int first = (warp - (int)u) & 3;                 // this warp's rows: first, first + 4, ...
+            const int nj = (first < R) ? (R - first + 3) >> 2 : 0;
+            const double sh = a.shift ? a.shift[g / a.nc] : 0.0;
+            // 2^(-(d*sc)^2) = exp(-d^2 / (2 h^2))
+            const float sc = (n > 0) ? (float)(0.8493218002880191 / a.h[g]) : 0.f;  // sqrt(log2(e)/2) / h
+            float qhi[4], qlo[4];
+            double acc[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int64_t qi = q0 + 32 * (first + 4 * j) + lane;
+                const double lq = log(fmax((j < nj && qi < q1) ? a.q_rt[qi] - sh : 1.0, a.eps));
+                qhi[j] = (float)lq;
+                qlo[j] = (float)(lq - (double)qhi[j]);
+                acc[j] = 0.0;
+            }
+            for (int64_t t = t0; t < t1 && n > 0; ++t) {
+                const int64_t b0 = t * KDE_TILE;
+                const int cnt = (int)min((int64_t)KDE_TILE, n - b0), n32 = (cnt + 31) >> 5;
+                __syncthreads();
+                for (int i = threadIdx.x; i < 32 * n32; i += KDE_THREADS)
+                    tile[i] = (i < cnt) ? __ldg(a.points + p0 + b0 + i) : 1e30f;  // padding: zero weight
+                __syncthreads();
+                switch (nj) {
+                    case 4: kde_tile<4>(tile, n32, qhi, qlo, sc, acc); break;
+                    case 3: kde_tile<3>(tile, n32, qhi, qlo, sc, acc); break;
+                    case 2: kde_tile<2>(tile, n32, qhi, qlo, sc, acc); break;
+                    case 1: kde_tile<1>(tile, n32, qhi, qlo, sc, acc); break;
+                    default: break;
+                }
+            }
+            const bool whole = (t0 == 0 && t1 == tiles);
+            // split unit: slot 0 if it began in an earlier CTA, else slot 1
+            double *slot = a.slots + (c * 2 + (t0 > 0 ? 0 : 1)) * KDE_QT;
+            if (!whole && t0 == 0) tail = (int)u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (j >= nj) continue;
+                const int r = 32 * (first + 4 * j) + lane;
+                const int64_t qi = q0 + r;
+                if (!whole) {
+                    slot[r] = acc[j];
+                } else if (qi < q1) {
                     const double disp = a.q_rt[qi] - sh;
                     a.out[qi] = kde_finalize(a, g, n, acc[j], disp, log(fmax(disp, a.eps)));
                 }
             }
-        } else {
-            // split unit: slot 0 (head) if it began in an earlier CTA, else slot 1 (tail)
-            double *slot = a.slots + (c * 2 + (ubeg < i0 ? 0 : 1)) * KDE_QT;
-#pragma unroll
-            for (int j = 0; j < KDE_QPT; ++j) slot[threadIdx.x + j * KDE_THREADS] = acc[j];
         }
-        it = hi;
-        ++u;
     }
+    if (threadIdx.x == 0) a.tail[c] = tail;
 }
 
-// Units split between CTAs: their partial sums are added in CTA order (a fixed
-// order, so results do not depend on timing) and finalised.
+// Units split between CTAs, one block per CTA that holds a first part: the
+// partial sums are added in CTA order (a fixed order, so results do not
+// depend on timing) and finalised.
 __global__ void __launch_bounds__(KDE_THREADS) k_kde_fixup(const KdeEval a) {
-    const int64_t U = min(a.uoff[a.G], a.u_max);
-    const int64_t I = a.ioff[a.u_max];
-    for (int64_t u = blockIdx.x; u < U; u += gridDim.x) {
-        const int64_t ubeg = a.ioff[u], uend = a.ioff[u + 1];
-        const int64_t c0 = sk_owner(ubeg, I, a.P), c1 = sk_owner(uend - 1, I, a.P);
-        if (c0 == c1) continue;
-        const int64_t g = upper_index(a.uoff, a.G + 1, u);
-        const int64_t q0 = a.qoff[g] + (u - a.uoff[g]) * KDE_QT, q1 = a.qoff[g + 1];
-        const int64_t n = a.poff[g + 1] - a.poff[g];
-        const double sh = a.shift ? a.shift[g / a.nc] : 0.0;
-        for (int j = 0; j < KDE_QPT; ++j) {
-            const int r = threadIdx.x + j * KDE_THREADS;
-            const int64_t qi = q0 + r;
-            if (qi >= q1) continue;
-            double acc = a.slots[(c0 * 2 + 1) * KDE_QT + r];
-            for (int64_t cc = c0 + 1; cc <= c1; ++cc)
-                if (sk_begin(cc, I, a.P) < sk_begin(cc + 1, I, a.P)) acc += a.slots[(cc * 2) * KDE_QT + r];
-            const double disp = a.q_rt[qi] - sh;
-            a.out[qi] = kde_finalize(a, g, n, acc, disp, log(fmax(disp, a.eps)));
+    const int64_t c = blockIdx.x;
+    const int u = a.tail[c];
+    if (u < 0) return;
+    const int64_t g = a.ugroup[u], qa = a.qoff[g], q1 = a.qoff[g + 1];
+    const UnitRows rows = unit_rows(q1 - qa, a.uidx[u]);
+    const int nq = 32 * (int)(rows.r1 - rows.r0);
+    const int64_t q0 = qa + 32 * rows.r0, n = a.poff[g + 1] - a.poff[g];
+    const double sh = a.shift ? a.shift[g / a.nc] : 0.0;
+    for (int r = threadIdx.x; r < nq; r += KDE_THREADS) {
+        const int64_t qi = q0 + r;
+        if (qi >= q1) continue;
+        double acc = a.slots[(c * 2 + 1) * KDE_QT + r];
+        bool more = true;
+        for (int64_t cc = c + 1; cc < a.P && more; cc += 4) {
+            int l[4];
+            double v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {  // four links and sums in flight
+                l[k] = (cc + k < a.P) ? a.link[cc + k] : SPLIT_LAST;
+                v[k] = (cc + k < a.P) ? a.slots[(cc + k) * 2 * KDE_QT + r] : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (more && l[k] != SPLIT_NONE) acc += v[k];
+                more = more && l[k] != SPLIT_LAST;
+            }
         }
+        const double disp = a.q_rt[qi] - sh;
+        a.out[qi] = kde_finalize(a, g, n, acc, disp, log(fmax(disp, a.eps)));
     }
 }
 
@@ -902,7 +1032,7 @@ static int64_t kde_eval_ctas() {
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct KdeEvalLayout {
-    size_t uoff, ucnt, ioff, icnt, slots, total;
+    size_t head, ioff, ugroup, uidx, tail, link, slots, total;
     int64_t u_max, P;
 };
 
@@ -910,11 +1040,13 @@ static KdeEvalLayout kde_eval_layout(int64_t G, int64_t n_queries) {
     KdeEvalLayout L;
     L.P = kde_eval_ctas();
     L.u_max = n_queries / KDE_QT + G + 1;
-    L.uoff = 0;
-    L.ucnt = L.uoff + align256((size_t)(G + 1) * 8);
-    L.ioff = L.ucnt + align256((size_t)G * 8);
-    L.icnt = L.ioff + align256((size_t)(L.u_max + 1) * 8);
-    L.slots = L.icnt + align256((size_t)L.u_max * 8);
+    L.head = 0;
+    L.ioff = L.head + 256;
+    L.ugroup = L.ioff + align256((size_t)(L.u_max + 1) * 8);
+    L.uidx = L.ugroup + align256((size_t)L.u_max * 4);
+    L.tail = L.uidx + align256((size_t)L.u_max * 4);
+    L.link = L.tail + align256((size_t)L.P * 4);
+    L.slots = L.link + align256((size_t)L.P * 4);
     L.total = L.slots + (size_t)L.P * 2 * KDE_QT * sizeof(double);
     return L;
 }
@@ -945,32 +1077,27 @@ int ssm_kde_eval(const float *points, const int64_t *point_offsets, const double
     SSM_REQUIRE(workspace_bytes >= L.total, "workspace too small: %zu bytes, need %zu (ssm_kde_eval_workspace_bytes)",
                 workspace_bytes, L.total);
     SSM_REQUIRE(((uintptr_t)workspace & 255) == 0, "workspace must be 256-byte aligned");
+    SSM_REQUIRE(L.u_max < (int64_t)1 << 31, "too many groups for one launch");
     uint8_t *ws = static_cast<uint8_t *>(workspace);
     KdeEval a;
     a.points = points; a.poff = point_offsets; a.h = bandwidth; a.lognorm = log_norm;
     a.qoff = query_offsets; a.q_rt = query_rt; a.out = out_loglik; a.nc = n_choices; a.G = G;
     a.soff = sample_offsets; a.shift = displace; a.lb = lb; a.eps = eps; a.max_t = max_t;
-    a.uoff = reinterpret_cast<int64_t *>(ws + L.uoff);
-    a.ucnt = reinterpret_cast<int64_t *>(ws + L.ucnt);
+    a.head = reinterpret_cast<int64_t *>(ws + L.head);
     a.ioff = reinterpret_cast<int64_t *>(ws + L.ioff);
-    a.icnt = reinterpret_cast<int64_t *>(ws + L.icnt);
+    a.ugroup = reinterpret_cast<int32_t *>(ws + L.ugroup);
+    a.uidx = reinterpret_cast<int32_t *>(ws + L.uidx);
+    a.tail = reinterpret_cast<int32_t *>(ws + L.tail);
+    a.link = reinterpret_cast<int32_t *>(ws + L.link);
     a.u_max = L.u_max;
     a.slots = reinterpret_cast<double *>(ws + L.slots);
     a.P = L.P;
     cudaStream_t st = (cudaStream_t)stream;
-    const int ng = (int)std::min<int64_t>((G + 255) / 256, 4096);
-    k_kde_units<<<ng, 256, 0, st>>>(a);
-    SSM_CUDA(cudaGetLastError());
-    k_scan_i64<<<1, 1024, 0, st>>>(a.ucnt, G, a.uoff);
-    SSM_CUDA(cudaGetLastError());
-    const int nu = (int)std::min<int64_t>((L.u_max + 255) / 256, 4096);
-    k_kde_unit_iters<<<nu, 256, 0, st>>>(a);
-    SSM_CUDA(cudaGetLastError());
-    k_scan_i64<<<1, 1024, 0, st>>>(a.icnt, L.u_max, a.ioff);
+    k_kde_plan<<<1, 1024, 0, st>>>(a);
     SSM_CUDA(cudaGetLastError());
     k_kde_eval<<<(unsigned)L.P, KDE_THREADS, 0, st>>>(a);
     SSM_CUDA(cudaGetLastError());
-    k_kde_fixup<<<(unsigned)std::min<int64_t>(L.u_max, 65535), KDE_THREADS, 0, st>>>(a);
+    k_kde_fixup<<<(unsigned)L.P, KDE_THREADS, 0, st>>>(a);
     SSM_CUDA(cudaGetLastError());
     return SSM_OK;
 }

@@ -60,3 +60,37 @@ def test_chunk_and_slice_edges(cuda, choices, shift_r, shift_c):
 @pytest.mark.parametrize("n_sets", [1, 75, 150, 300, 700])
 def test_cluster_sizes(cuda, n_sets):
     _check(list(100 + (np.arange(n_sets) * 37) % 200), (-1, 1), 0, 0, n_sets)
+
+
+def test_evaluation_unit_and_tile_edges(cuda):
+    """Query counts around a row (32), a unit (512) and several units, point
+    counts around a staged tile (512) and the 32-term groups, empty groups on
+    either side: against the float64 sum over the fitted points, with the
+    tolerance of the KDE evaluation (1e-5 absolute plus 2e-6 relative)."""
+    rng = np.random.default_rng(3)
+    n_pts = [0, 1, 31, 32, 33, 511, 512, 513, 1025, 5000]
+    n_q = [0, 1, 31, 32, 33, 511, 512, 513, 1024, 1537]
+    pairs = [(p, q) for p in n_pts for q in n_q]
+    sizes = np.array([p for p, _ in pairs])
+    rts = np.exp(rng.normal(0.0, 0.5, int(sizes.sum()))).astype(np.float32)
+    soff = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    kb = gk.KdeBatch(torch.from_numpy(rts), torch.ones(rts.size, dtype=torch.int32), soff, [1])
+    qoff = np.concatenate([[0], np.cumsum([q for _, q in pairs])]).astype(np.int64)
+    q = np.exp(rng.normal(0.0, 0.8, int(qoff[-1])))
+    q[::97] = 0.0  # not after the start: the floor
+    ll = kb.evaluate(qoff, torch.from_numpy(q), max_t=20.0).cpu().numpy()
+    pts, h = kb.points.cpu().numpy().astype(np.float64), kb.bandwidth.cpu().numpy()
+    for g, (p, m) in enumerate(pairs):
+        got, qq = ll[qoff[g]:qoff[g + 1]], q[qoff[g]:qoff[g + 1]]
+        if p == 0:
+            with np.errstate(divide="ignore"):
+                np.testing.assert_array_equal(got, np.full(m, -np.log(np.float64(0.0) * 20.0)))
+            continue
+        lq = np.log(np.maximum(qq, 1e-4))
+        d = (lq[:, None] - pts[None, soff[g]:soff[g + 1]]) / h[g]
+        with np.errstate(divide="ignore"):
+            want = np.log(np.exp(-0.5 * d * d).sum(axis=1) / (p * h[g] * np.sqrt(2 * np.pi))) - lq
+        want = np.where((qq > 0) & (want > -66.774), want, -66.774)
+        floor = (got == -66.774) | (want == -66.774)
+        np.testing.assert_allclose(got[~floor], want[~floor], rtol=2e-6, atol=1e-5)
+        assert np.all(np.abs(got - want)[floor] < 1e-3)
