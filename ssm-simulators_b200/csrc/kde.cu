@@ -27,6 +27,7 @@
 namespace ssm {
 
 constexpr int KDE_MAX_CHOICES = 16;
+constexpr int KDE_MAX_ROWS = 12288;  // records per set
 constexpr double KDE_LOG_2PI = 1.8378770664093453;
 
 struct KdeFit {
@@ -818,25 +819,53 @@ struct KdeRecords {
     float *out;      // [S * rows_per_set, P + 3]
 };
 
+// The Fisher-Yates shuffle "for i = M-1 .. 1: swap(perm[i], perm[j_i])" in
+// parallel rounds with the result of the sequential loop (deterministic
+// reservations: Shun, Gu, Blelloch, Fineman & Gibbons, SODA'15): every swap not
+// yet done bids for its two places, the earliest swap (largest i) wins a place,
+// and a swap that won both is done.  About log M rounds instead of M dependent
+// swaps by one thread: 256 sets of 1 000 rows, 137 -> 27 us.
 __global__ void __launch_bounds__(256) k_kde_records(const KdeRecords a) {
-    extern __shared__ int perm[];
+    extern __shared__ int bid[];  // [M] bids, then [M] 16-bit places and [M] 16-bit partners
     const int64_t s = blockIdx.x;
-    const int64_t M = a.rows_per_set;
+    const int M = (int)a.rows_per_set;
+    uint16_t *perm = reinterpret_cast<uint16_t *>(bid + M), *other = perm + M;
     const int64_t qa = a.qoff[s * a.nc], qb = a.qoff[(s + 1) * a.nc];
-    for (int64_t i = threadIdx.x; i < M; i += blockDim.x) perm[i] = (int)i;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int64_t i = M - 1; i > 0; --i) {
-            const uint4 r = philox10(make_uint4((uint32_t)i, (uint32_t)s, (uint32_t)(s >> 32), 9u), a.key);
-            const int64_t j = (int64_t)(u53(r.x, r.y) * (double)(i + 1));
-            const int tmp = perm[i];
-            perm[i] = perm[j <= i ? j : i];
-            perm[j <= i ? j : i] = tmp;
-        }
+    for (int i = threadIdx.x; i < M; i += blockDim.x) {
+        const uint4 r = philox10(make_uint4((uint32_t)i, (uint32_t)s, (uint32_t)(s >> 32), 9u), a.key);
+        const int j = (int)(u53(r.x, r.y) * (double)(i + 1));
+        perm[i] = (uint16_t)i;
+        other[i] = (uint16_t)(j <= i ? j : i);
+        bid[i] = 0;
     }
+    // this thread's swaps i = threadIdx.x + k blockDim.x not yet done, one bit each (i = 0 is none)
+    static_assert(KDE_MAX_ROWS <= 64 * 256, "one bit per swap of a thread");
+    unsigned long long open = 0ull;
+    for (int i = threadIdx.x, k = 0; i < M; i += blockDim.x, ++k)
+        if (i > 0) open |= 1ull << k;
     __syncthreads();
+    for (int round = 1;; ++round) {
+        // a later round's bids beat all earlier ones, so nothing is cleared (M < 2^14, rounds <= M)
+        for (unsigned long long m = open; m; m &= m - 1) {
+            const int i = threadIdx.x + (__ffsll((long long)m) - 1) * (int)blockDim.x;
+            atomicMax(&bid[i], (round << 14) | i);
+            atomicMax(&bid[other[i]], (round << 14) | i);
+        }
+        __syncthreads();
+        for (unsigned long long m = open; m; m &= m - 1) {
+            const int k = __ffsll((long long)m) - 1, i = threadIdx.x + k * (int)blockDim.x, j = other[i];
+            const int mine = (round << 14) | i;
+            if (bid[i] == mine && bid[j] == mine) {
+                const uint16_t t = perm[i];
+                perm[i] = perm[j];
+                perm[j] = t;
+                open &= ~(1ull << k);
+            }
+        }
+        if (!__syncthreads_or(open != 0ull)) break;
+    }
     const int W = a.P + 3;
-    for (int64_t i = threadIdx.x; i < M; i += blockDim.x) {
+    for (int i = threadIdx.x; i < M; i += blockDim.x) {
         float *row = a.out + (s * M + perm[i]) * W;
         for (int p = 0; p < a.P; ++p) row[p] = a.theta[s * a.P + p];
         float rt, ch, ll;
@@ -868,6 +897,7 @@ __global__ void __launch_bounds__(256) k_kde_records(const KdeRecords a) {
 struct SetSummary {
     const float *rts;
     const int32_t *choices;
+    int64_t n_sets;
     const int64_t *soff;
     const int32_t *cvals;
     int nc;
@@ -877,59 +907,103 @@ struct SetSummary {
     float *hist_a, *hist_b;
 };
 
-__device__ __forceinline__ int np_hist_index(double v, double max_t, int nb) {
+// numpy.histogram's bin of v over linspace(0, max_t, nb + 1) (step = max_t / nb
+// in float64): the i with i step <= v < (i + 1) step, the last bin closed; -1
+// outside.  A float32 guess, then moved to the bin whose float64 edges hold v.
+__device__ __forceinline__ int np_hist_index(float rt, double max_t, double step, float inv_step, int nb) {
+    const double v = (double)rt;
     if (!(v >= 0.0) || !(v <= max_t)) return -1;
-    const double step = max_t / (double)nb;
-    int i = (int)((v / max_t) * (double)nb);
-    if (i == nb) i -= 1;
-    const double lo = (double)i * step;
-    if (v < lo) i -= 1;
-    const double hi = (i + 1 == nb) ? max_t : (double)(i + 1) * step;
-    if (i != nb - 1 && v >= hi) i += 1;
+    int i = max(min((int)(rt * inv_step), nb - 1), 0);
+    while (i > 0 && v < (double)i * step) --i;
+    while (i < nb - 1 && v >= (double)(i + 1) * step) ++i;
     return i;
 }
 
+// One pass over a set's samples by its cluster: counts in registers, the
+// histograms as 32-bit shared counters per CTA (equal bins of a warp are added
+// up by the hardware), added over the cluster at the end.  A histogram with half
+// the bins of the other is its pairwise sum (its edges are every second one,
+// exactly: the steps differ by a power of two).  64-bit shared counters hit by
+// every lane and two float64 divisions per sample: 256 sets of 50 000 samples
+// 2 176 -> 50 us.
+template <int NC>
 __global__ void __launch_bounds__(256) k_set_summary(const SetSummary a) {
+    namespace cg = cooperative_groups;
     extern __shared__ unsigned int sh[];  // [nc * (nb_a + nb_b)] histogram counters
-    __shared__ unsigned long long cnt[KDE_MAX_CHOICES];
-    __shared__ unsigned long long nogo, omit;
-    const int64_t s = blockIdx.x;
+    __shared__ unsigned int cnt[NC + 2];  // choices, no-go, omissions
+    cg::cluster_group cl = cg::this_cluster();
+    const Slice sl = set_slice(a.soff, a.n_sets);
+    const ChoiceSet<NC> cs(a.cvals, a.nc);
     const int H = a.nc * (a.nb_a + a.nb_b);
-    int32_t max_choice = __ldg(a.cvals);
-    for (int c = 1; c < a.nc; ++c) max_choice = max(max_choice, __ldg(a.cvals + c));
+    const bool pairs = (a.nb_b == 2 * a.nb_a);
+    const double step_a = a.max_t / (double)a.nb_a, step_b = a.max_t / (double)a.nb_b;
+    const float inv_a = (float)(1.0 / step_a), inv_b = (float)(1.0 / step_b);
+    unsigned int *hb = sh + a.nc * a.nb_a;
+    int32_t max_choice = cs.v[0];
+#pragma unroll
+    for (int c = 1; c < NC; ++c)
+        if (c < a.nc) max_choice = max(max_choice, cs.v[c]);
     for (int i = threadIdx.x; i < H; i += blockDim.x) sh[i] = 0u;
-    if (threadIdx.x < KDE_MAX_CHOICES) cnt[threadIdx.x] = 0ull;
-    if (threadIdx.x == 0) nogo = omit = 0ull;
+    if (threadIdx.x < NC + 2) cnt[threadIdx.x] = 0u;
     __syncthreads();
-    for (int64_t i = a.soff[s] + threadIdx.x; i < a.soff[s + 1]; i += blockDim.x) {
-        const int32_t ch = a.choices[i];
-        const float rt = a.rts[i];
-        if (ch == -999) atomicAdd(&omit, 1ull);
-        if (ch != max_choice || rt == -999.f) atomicAdd(&nogo, 1ull);
-        const int c = choice_index(ch, a.cvals, a.nc);
-        if (c < 0) continue;
-        atomicAdd(&cnt[c], 1ull);
-        if (rt == -999.f) continue;
-        const int ia = np_hist_index((double)rt, a.max_t, a.nb_a);
-        if (ia >= 0) atomicAdd(&sh[c * a.nb_a + ia], 1u);
-        const int ib = np_hist_index((double)rt, a.max_t, a.nb_b);
-        if (ib >= 0) atomicAdd(&sh[a.nc * a.nb_a + c * a.nb_b + ib], 1u);
+    unsigned int n[NC], nogo = 0u, omit = 0u;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) n[c] = 0u;
+    for_each_sample(a.rts, a.choices, sl.lo, sl.hi, [&](float rt, int32_t ch) {
+        const bool omitted = (rt == -999.f);
+        omit += (ch == -999);
+        nogo += (ch != max_choice || omitted);
+        const int c = cs.index(ch);
+#pragma unroll
+        for (int k = 0; k < NC; ++k) n[k] += (c == k);
+        if (c < 0 || omitted) return;
+        const int ib = np_hist_index(rt, a.max_t, step_b, inv_b, a.nb_b);
+        if (ib >= 0) atomicAdd(&hb[c * a.nb_b + ib], 1u);
+        if (!pairs) {
+            const int ia = np_hist_index(rt, a.max_t, step_a, inv_a, a.nb_a);
+            if (ia >= 0) atomicAdd(&sh[c * a.nb_a + ia], 1u);
+        }
+    });
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const unsigned int x = __reduce_add_sync(0xffffffffu, n[c]);
+        if (lane == 0 && c < a.nc) atomicAdd(&cnt[c], x);
     }
-    __syncthreads();
-    if (threadIdx.x < a.nc) a.counts[s * a.nc + threadIdx.x] = (int64_t)cnt[threadIdx.x];
-    if (threadIdx.x == 0) {
-        a.nogo[s] = (int64_t)nogo;
-        a.omit[s] = (int64_t)omit;
+    nogo = __reduce_add_sync(0xffffffffu, nogo);
+    omit = __reduce_add_sync(0xffffffffu, omit);
+    if (lane == 0) {
+        atomicAdd(&cnt[NC], nogo);
+        atomicAdd(&cnt[NC + 1], omit);
     }
-    // layout [S, nb, nc] like the pipeline's binned_128 / binned_256 arrays
-    for (int i = threadIdx.x; i < a.nc * a.nb_a; i += blockDim.x) {
-        const int c = i / a.nb_a, b = i % a.nb_a;
-        a.hist_a[(s * a.nb_a + b) * a.nc + c] = (float)sh[i];
+    if (pairs) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < a.nc * a.nb_a; i += blockDim.x) {
+            const int c = i / a.nb_a, k = i - c * a.nb_a;
+            sh[i] = hb[c * a.nb_b + 2 * k] + hb[c * a.nb_b + 2 * k + 1];
+        }
     }
-    for (int i = threadIdx.x; i < a.nc * a.nb_b; i += blockDim.x) {
-        const int c = i / a.nb_b, b = i % a.nb_b;
-        a.hist_b[(s * a.nb_b + b) * a.nc + c] = (float)sh[a.nc * a.nb_a + i];
+    cl.sync();
+    if (sl.rank == 0 && threadIdx.x < NC + 2) {
+        int64_t x = 0;
+        for (unsigned j = 0; j < sl.J; ++j) x += cl.map_shared_rank(cnt, j)[threadIdx.x];
+        if ((int)threadIdx.x < a.nc) a.counts[sl.set * a.nc + threadIdx.x] = x;
+        if (threadIdx.x == NC) a.nogo[sl.set] = x;
+        if (threadIdx.x == NC + 1) a.omit[sl.set] = x;
     }
+    // layout [S, nb, nc] like the pipeline's binned_128 / binned_256 arrays; the ranks share the bins
+    for (int i = (int)sl.rank * (int)blockDim.x + threadIdx.x; i < H; i += (int)(sl.J * blockDim.x)) {
+        int64_t x = 0;
+        for (unsigned j = 0; j < sl.J; ++j) x += cl.map_shared_rank(sh, j)[i];
+        if (i < a.nc * a.nb_a) {
+            const int c = i / a.nb_a, b = i % a.nb_a;
+            a.hist_a[(sl.set * a.nb_a + b) * a.nc + c] = (float)x;
+        } else {
+            const int k = i - a.nc * a.nb_a, c = k / a.nb_b, b = k % a.nb_b;
+            a.hist_b[(sl.set * a.nb_b + b) * a.nc + c] = (float)x;
+        }
+    }
+    cl.sync();  // the others' counters stay until they have been read
 }
 
 // CTAs per set of the per-set kernels (a cluster, at most the portable 8): the
@@ -984,13 +1058,16 @@ int ssm_set_summary(const float *rts, const int32_t *choices, int64_t n_sets,
     SSM_REQUIRE(rts && choices && sample_offsets && choice_values && choice_counts && nogo_counts &&
                 omission_counts && hist_a && hist_b, "all buffers are required");
     SetSummary a;
+    a.n_sets = n_sets;
     a.rts = rts; a.choices = choices; a.soff = sample_offsets; a.cvals = choice_values;
     a.nc = n_choices; a.max_t = max_t; a.counts = choice_counts; a.nogo = nogo_counts;
     a.omit = omission_counts; a.nb_a = nbins_a; a.nb_b = nbins_b; a.hist_a = hist_a; a.hist_b = hist_b;
     const size_t smem = (size_t)n_choices * (nbins_a + nbins_b) * sizeof(unsigned int);
-    k_set_summary<<<(unsigned)n_sets, 256, smem, (cudaStream_t)stream>>>(a);
-    SSM_CUDA(cudaGetLastError());
-    return SSM_OK;
+    SSM_REQUIRE(n_sets < (int64_t)1 << 28, "too many sets for one launch");
+    cudaStream_t st = (cudaStream_t)stream;
+    if (n_choices <= 2) return launch_per_set(k_set_summary<2>, a, n_sets, smem, st);
+    if (n_choices <= 4) return launch_per_set(k_set_summary<4>, a, n_sets, smem, st);
+    return launch_per_set(k_set_summary<KDE_MAX_CHOICES>, a, n_sets, smem, st);
 }
 
 int ssm_kde_fit(const float *rts, const int32_t *choices, int64_t n_sets,
@@ -1127,7 +1204,7 @@ int ssm_kde_records(const float *theta, int n_params, int64_t n_sets, int n_choi
                     void *stream) {
     using namespace ssm;
     SSM_REQUIRE(n_sets >= 0 && n_params >= 1 && n_choices >= 1 && n_choices <= KDE_MAX_CHOICES, "bad sizes");
-    SSM_REQUIRE(rows_per_set >= 1 && rows_per_set <= 12288, "rows_per_set must be in [1, 12288]");
+    SSM_REQUIRE(rows_per_set >= 1 && rows_per_set <= KDE_MAX_ROWS, "rows_per_set must be in [1, %d]", KDE_MAX_ROWS);
     if (n_sets == 0) return SSM_OK;
     SSM_REQUIRE(theta && choice_values && query_offsets && query_rt && query_loglik && out, "all buffers are required");
     KdeRecords a;
@@ -1135,7 +1212,10 @@ int ssm_kde_records(const float *theta, int n_params, int64_t n_sets, int n_choi
     a.theta = theta; a.P = n_params; a.n_sets = n_sets; a.qoff = query_offsets; a.q_rt = query_rt;
     a.q_ll = query_loglik; a.cvals = choice_values; a.nc = n_choices; a.n_down = n_down;
     a.rows_per_set = rows_per_set; a.neg_ll = negative_rt_loglik; a.out = out;
-    k_kde_records<<<(unsigned)n_sets, 256, rows_per_set * sizeof(int), (cudaStream_t)stream>>>(a);
+    const size_t smem = (size_t)rows_per_set * (sizeof(int) + 2 * sizeof(uint16_t));
+    if (smem > 48 * 1024)
+        SSM_CUDA(cudaFuncSetAttribute(k_kde_records, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_kde_records<<<(unsigned)n_sets, 256, smem, (cudaStream_t)stream>>>(a);
     SSM_CUDA(cudaGetLastError());
     return SSM_OK;
 }
