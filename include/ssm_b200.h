@@ -52,7 +52,7 @@ extern "C" {
 typedef struct ssm_launch {
     int block_threads;     /* 0 = library default (autotuned value if set) */
     int blocks_per_sm;     /* 0 = as many as fit                            */
-    int chunk;             /* trajectories a warp claims per queue access; 0 = default */
+    int chunk;             /* most trajectories a warp claims per queue access; 0 = default */
     int refill_min;        /* ended walks a warp collects before restarting lanes (1-32); 0 = default */
     /* Index that trial 0 of this call has in the random streams (0 = none).
      * A batch simulated as several calls over consecutive trial windows --
@@ -73,12 +73,15 @@ typedef struct ssm_launch {
     const int32_t *trial_order;
     const int64_t *order_offsets;
     /* Lanes per trajectory of the single-accumulator simulators (device RNG,
-     * constant / linear / Weibull boundary): 1, 2, 4 or 8; 0 = automatic,
+     * constant / linear / Weibull boundary): 1, 2, 4, 8, 16 or 32; 0 = automatic,
      * which is 1 for the ragged layout and otherwise chosen from the number
      * of trajectories against the grid's lanes (ssm_auto_lanes_per_walk).
-     * With W > 1 the W lanes of a group draw a walk's increments in parallel
-     * and step it together: results are bit-identical to W = 1, and a launch
-     * with fewer trajectories than lanes ends sooner; chunk is 32 / W. */
+     * With W >= 8 the lanes of a group draw a walk's increments in parallel and
+     * share its tests: results are bit-identical to W = 1, and a launch
+     * with fewer trajectories than lanes ends sooner; chunk is 32 / W.  The
+     * library may take more lanes than asked for where the number of
+     * trajectories is small, and one lane (with the launch's last trajectories
+     * on several) for 2 and 4, which gained nothing over that. */
     int lanes_per_walk;
 } ssm_launch;
 
@@ -92,7 +95,10 @@ int ssm_check_status(const void *workspace, void *stream);
 
 /* ---- single-accumulator Euler-Maruyama DDM family ----------------------- */
 
-/* Bytes of scratch the DDM-family entry points need for n_trials trials. */
+/* Bytes of scratch for the DDM-family entry points with n_trials trials: 256 B +
+ * 64 B a trial, which they require, and room for the walks that a launch of one
+ * lane per walk leaves to several lanes at its end (7.3 MB on 148 SMs; a smaller
+ * workspace is accepted, and the launch then ends on one lane per walk). */
 size_t ssm_ddm_workspace_bytes(int64_t n_trials);
 /* Lanes per walk (ssm_launch.lanes_per_walk) the library picks for a
  * single-accumulator launch of n_walks trajectories on the current device

@@ -29,28 +29,28 @@ int sm_count();
     } while (0)
 
 // Trajectories a persistent simulator warp claims per queue access: the
-// caller's chunk, cut (to a multiple of the warp's walk slots -- 32, or 32 / W
-// with W lanes per walk -- and at least one slot per walk) so that every warp
-// of the grid gets work when the launch is small.
-__device__ __forceinline__ int64_t warp_chunk(int chunk, int64_t total, int slots = 32) {
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    const int64_t fair = ((total + warps - 1) / warps + slots - 1) / slots * slots;
-    return max((int64_t)slots, min((int64_t)chunk, fair));
+// caller's chunk, cut to a twelfth of a warp's share of the launch (a multiple
+// of the warp's 32 walks, at least one each), so that no warp is left with a large
+// claim at the end, nor with a large one of the longest walks, which come first.
+// Measured with claims of 256 / 64 (ms): 256 angle sets 2.62 / 1.67, 64 sets
+// 1.48 / 0.84, 4 096 sets 23.8 / 24.1.
+__device__ __forceinline__ int64_t warp_chunk(int chunk, int64_t total) {
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5) * 12;
+    const int64_t fair = ((total + warps - 1) / warps + 31) / 32 * 32;
+    return max((int64_t)32, min((int64_t)chunk, fair));
 }
 
 // Ended walks a persistent simulator warp collects before it writes their
 // results and restarts those lanes (ssm_launch.refill_min = 0).  Batching
-// pays where a step is cheap next to the restart (single accumulator, 4:
-// 10-12 % faster than 1 on the angle and full_ddm batches).  The race kernel,
-// whose steps cost more, restarts two at a time by default: with windows of
-// steps drawn ahead, 1 024-set launches measured 2.4 % (LCA) and 7.9 %
-// (racing diffusion) faster with 2 than with 1, and the race model 8.3 %
-// with 6 (its tuned value, like the others', is in the launch-option store).
+// pays where a step is cheap next to the restart.  Measured defaults: with restarts
+// that stay in their trial two at a time are best on the single-accumulator
+// batches (4 096 angle sets: 24.3 ms, four 24.5), four on the race family (racing
+// diffusion 9.7 ms, two 9.9; LCA 15.1, 15.3).
 #ifndef SSM_REFILL_MIN
-#define SSM_REFILL_MIN 4
+#define SSM_REFILL_MIN 2
 #endif
 #ifndef SSM_REFILL_MIN_RACE
-#define SSM_REFILL_MIN_RACE 2
+#define SSM_REFILL_MIN_RACE 4
 #endif
 
 // Workspace header shared by every persistent kernel: a work counter and an
@@ -129,6 +129,35 @@ __device__ __forceinline__ void sincos_ftz(float x, float &s, float &c) {
     asm("cos.approx.ftz.f32 %0, %1;" : "=f"(c) : "f"(x));
 }
 
+// Packed pairs of float32: two IEEE operations per instruction with the results
+// of the scalar ones.  The simulators and the KDE are bound by issue slots or the
+// SFU, not by the FP32 lanes, so a packed operation saves an issue slot.
+__device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack_f2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul_f2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // Box-Muller transform of two 32-bit words into two N(0,1) variates
 // (r = sqrt(-2 ln u1), phase 2 pi u2).  Uses the SFU approximations of log2,
 // rsqrt, sin and cos: 4 MUFU operations per pair (u1 >= 2^-24 and the phase
@@ -141,6 +170,15 @@ __device__ __forceinline__ float2 box_muller(uint32_t a, uint32_t b) {
     float s, c;
     sincos_ftz(6.2831853f * u2, s, c);
     return make_float2(r * c, r * s);
+}
+
+// The top nine bits of hi and of lo as an 18-bit phase in the upper bits of a
+// float mantissa (bits 22-14 and 13-5): one shift, one funnel shift and the mask
+// (which joins the exponent's OR), where two shifts and two masks would be four.
+// The ALU pipe takes two cycles an instruction and an added one cost the angle
+// batch 1.6 ms per step; this is one instruction less per pair.
+__device__ __forceinline__ uint32_t phase18(uint32_t hi, uint32_t lo) {
+    return __funnelshift_r(lo, hi >> 23, 18) & 0x007fffe0u;
 }
 
 // Six increments from one Philox4x32-10 call (128 bits): three Box-Muller pairs whose
@@ -156,8 +194,7 @@ __device__ __forceinline__ float2 box_muller(uint32_t a, uint32_t b) {
 __device__ __forceinline__ void bm6_increment_pairs(uint4 b, const float (&c2)[3], const float (&drift)[3],
                                                     float *g) {
     const uint32_t rad[3] = {b.x, b.y, b.z};
-    const uint32_t ph[3] = {b.w & 0x007fffffu, ((b.w >> 9) & 0x7fc000u) | ((b.x >> 18) & 0x3fe0u),
-                            ((b.y >> 9) & 0x7fc000u) | ((b.z >> 18) & 0x3fe0u)};
+    const uint32_t ph[3] = {b.w & 0x007fffffu, phase18(b.w, b.x), phase18(b.y, b.z)};
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const float u1 = __uint_as_float(0x3f800000u | (rad[i] & 0x007fffffu)) - 0.99999994f;  // (0, 1)
@@ -174,6 +211,48 @@ __device__ __forceinline__ void bm6_increment_pairs(uint4 b, const float (&c2)[3
 __device__ __forceinline__ void bm6_increment(uint4 b, float c2, float drift, float *g) {
     const float c[3] = {c2, c2, c2}, d[3] = {drift, drift, drift};
     bm6_increment_pairs(b, c, d, g);
+}
+
+// Two Box-Muller pairs (bits ra, pa and rb, pb; radius constants c2, drifts d) with
+// the FP32 operations packed: cs and sn hold pair a's output in the lower half,
+// pair b's in the upper one, the values of bm6_increment_pairs.
+__device__ __forceinline__ void bm_pair2(uint32_t ra, uint32_t rb, uint32_t pa, uint32_t pb, uint64_t c2,
+                                         uint64_t d, uint64_t &cs, uint64_t &sn) {
+    const float2 u = unpack_f2(add_f2(pack_f2(__uint_as_float(0x3f800000u | (ra & 0x007fffffu)),
+                                              __uint_as_float(0x3f800000u | (rb & 0x007fffffu))),
+                                      pack_f2(-0.99999994f, -0.99999994f)));
+    const float2 ang = unpack_f2(fma_f2(pack_f2(__uint_as_float(0x3f800000u | pa), __uint_as_float(0x3f800000u | pb)),
+                                        pack_f2(6.2831853f, 6.2831853f), pack_f2(-6.2831853f, -6.2831853f)));
+    const float2 e = unpack_f2(mul_f2(c2, pack_f2(lg2_ftz(u.x), lg2_ftz(u.y))));
+    float r0, r1, s0, s1, k0, k1;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(e.x));
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(e.y));
+    sincos_ftz(ang.x, s0, k0);
+    sincos_ftz(ang.y, s1, k1);
+    const uint64_t r = pack_f2(r0, r1);
+    cs = fma_f2(r, pack_f2(k0, k1), d);
+    sn = fma_f2(r, pack_f2(s0, s1), d);
+}
+
+// Twelve increments from two calls, two Box-Muller pairs to an instruction
+// wherever the arithmetic is FP32 (7.5 issue slots fewer per six increments than
+// bm6_increment_pairs, the same values): pairs (0, 1), (2, 3), (4, 5) of the six
+// share the packed operations, the SFU ones stay scalar.
+__device__ __forceinline__ void bm12_increment(uint4 b0, uint4 b1, float c2, float drift, float *g) {
+    const uint32_t rad[6] = {b0.x, b0.y, b0.z, b1.x, b1.y, b1.z};
+    const uint32_t ph[6] = {b0.w & 0x007fffffu, phase18(b0.w, b0.x), phase18(b0.y, b0.z),
+                            b1.w & 0x007fffffu, phase18(b1.w, b1.x), phase18(b1.y, b1.z)};
+    const uint64_t c = pack_f2(c2, c2), d = pack_f2(drift, drift);
+#pragma unroll
+    for (int i = 0; i < 6; i += 2) {
+        uint64_t cs, sn;
+        bm_pair2(rad[i], rad[i + 1], ph[i], ph[i + 1], c, d, cs, sn);
+        const float2 k = unpack_f2(cs), s = unpack_f2(sn);
+        g[2 * i] = k.x;
+        g[2 * i + 1] = s.x;
+        g[2 * i + 2] = k.y;
+        g[2 * i + 3] = s.y;
+    }
 }
 
 __device__ __forceinline__ void raise_error(WorkspaceHeader *h, int code, int detail) {

@@ -13,16 +13,24 @@
 //    divergent pass, so that pass is paid once per several trajectories and
 //    an ended lane idles for a few blocks at most.
 //  * Steps run in blocks of 36 (24 for ddm_flex with a Weibull or table
-//    bound, 8 for Levy): six independent Philox4x32-10 calls yield 24 words =
+//    bound, 16 for Levy): six independent Philox4x32-10 calls yield 24 words =
 //    18 Box-Muller pairs = the block's increments, already scaled to drift +
-//    s sqrt(dt) N(0,1), each call drawn in the step loop just before the six
-//    steps that use it; the steps themselves are predicated (no per-step
-//    branch), and a warp whose walks cannot reach their time limit within the
-//    block skips the time test.
-//  * A launch with about as many trajectories as the grid has lanes lasts as
-//    long as its longest walk.  There W = 2, 4 or 8 lanes share a walk
-//    (ssm_launch.lanes_per_walk, wide_block): each draws a third of the
-//    block's increments and all step it, bit-identical to one lane per walk.
+//    s sqrt(dt) N(0,1), drawn two calls at a time in the step loop just before
+//    the twelve steps that use them, with two pairs to an FP32 instruction; the
+//    steps themselves are predicated (no per-step branch), and a warp whose walks
+//    cannot reach their time limit within the block skips the time test.
+//  * What bounds it: the issue of integer and SFU work of the draws.  A step
+//    of the angle batch takes 26 cycles of a warp scheduler; its SFU operations alone
+//    (two per increment, eight cycles each) 16.  Occupancy does not matter from 8
+//    warps per SM up.  4 096 angle sets, 43 M walks: 27.4 -> 24.3 ms (packed pairs,
+//    the rts turned from times into results by k_finish, restarts that stay in
+//    their trial without a search); 509 Levy sets of 9 973: 19.1 -> 14.5 ms (packed
+//    transform, 16-step blocks).
+//  * A launch lasts as long as its longest walk.  When the queue is empty and a
+//    warp has at most LEAVE_MAX walks left, it hands them (LeftWalk) to k_wide
+//    (sim_wide.cu), which gives a walk 8 to 32 lanes; a launch with fewer walks
+//    than the grid has lanes goes there as a whole (ssm_launch.lanes_per_walk).
+//    Outputs are bit-identical to one lane per walk.
 //  * Boundaries are evaluated in registers (constant / linear collapse /
 //    Weibull) or read from a caller-evaluated table for arbitrary shapes.
 //  * Noise injection replaces the generator by caller rows and switches every
@@ -30,71 +38,12 @@
 //    bit-identical to the sequential CPU restatement.
 #include <cuda.h>  // CUcontext / CUresult types of the driver entry points below
 
+#include <algorithm>
 #include <mutex>
 
-#include "common.cuh"
-
-
-
-
+#include "sim_single.cuh"
 
 namespace ssm {
-
-// M_SDV: ddm_sdv (drift v + sv N(0,1) per trajectory); M_FULL: full_ddm (and
-// start point + U(-sz, sz), non-decision time + U(-st, st)); M_OU:
-// ornstein_uhlenbeck (drift v - g y); M_DFLEX: ddm_flex (drift v(t) from a
-// per-trial table the host evaluates from the drift function).
-enum Model { M_FLEX = 0, M_LEGACY = 1, M_LEVY = 2, M_SDV = 3, M_FULL = 4, M_OU = 5, M_DFLEX = 6 };
-
-struct alignas(16) TrialRow {
-    float drift;     // v * dt ; SDV/FULL: v
-    float scale;     // sqrt(dt) * s ;  Levy: s * dt^(1/alpha)
-    float y0;        // start point
-    float dl_tmp;    // min(max_t, deadline - t): the walk runs while t <= dl_tmp
-    float t;         // non-decision time
-    float deadline;  // rt >= deadline (or deadline <= 0) -> omission
-    float a;         // boundary height (legacy DDM: upper bound)
-    float p1;        // LINEAR: slope ; WEIBULL: shape alpha
-    float p2;        // WEIBULL: scale beta
-    float dtp1;      // dt * p1 (linear boundary per step, fast path)
-    float inv_beta;  // 1 / beta
-    float alpha;     // Levy: stability index ; SDV/FULL: sv ; OU: v
-    float inv_alpha; // Levy: 1 / alpha ; FULL: sz ; OU: g
-    float expo;      // Levy: (1 - alpha) / alpha ; FULL: st ; OU: 1 - g dt
-    float capf;      // hard limit on Euler steps: a walk reaching it raises SSM_ERR_DEVICE
-    float c2;        // -2 ln(2) * scale^2: folds the noise scale into Box-Muller's radius
-};
-static_assert(sizeof(TrialRow) == 64, "TrialRow is one 64-byte line");
-
-struct SingleParams {
-    PhiloxKeys key;
-    const TrialRow *rows;
-    const int64_t *offsets;  // ragged prefix sums (n_trials + 1) or nullptr
-    const int32_t *order;    // ragged only: trial simulated j-th (nullptr = index order)
-    const int64_t *qoff;     // prefix sums of the sample counts in that order
-    int64_t n_trials;
-    int64_t total;           // number of trajectories; -1 = offsets[n_trials] - offsets[0]
-    uint32_t k_base;         // random-stream index of trial 0 (trial windows of a larger batch)
-    int ustride;             // injected uniforms per trajectory (3 for full_ddm: u_t, u_y, u_smooth)
-    float dt;
-    int smooth;
-    int chunk;
-    int refill_min;          // ended walks a warp collects before it restarts lanes
-    const float *table;
-    int64_t tstride, tlen;
-    const float *dtable;     // DFLEX: drift v(t_ix) per trial, row stride dstride, dlen entries
-    int64_t dstride, dlen;
-    int dvec;                // rows 16-byte aligned: a block's drifts are float4 loads
-    const float *noise;      // injected increments: row w holds nlen floats
-    int64_t nlen;
-    const float *nunif;      // injected jitter uniforms, one per trajectory
-    float *rts;
-    int32_t *choices;
-    int32_t *steps;
-    WorkspaceHeader *hdr;
-    float *traj;             // trajectory recorder (record kernel only)
-    int64_t traj_len;
-};
 
 struct PrepArgs {
     const float *v, *a, *z, *t, *deadline, *s, *alpha, *p1, *p2, *maxt_k, *table;
@@ -165,106 +114,6 @@ __global__ void k_prep(const PrepArgs A) {
     reinterpret_cast<TrialRow *>(A.rows)[k] = r;
 }
 
-// ------------------------------------------------------------------ helpers
-__device__ __forceinline__ int64_t ragged_find(const int64_t *off, int64_t K, int64_t w,
-                                               int64_t hint) {
-    int64_t k = hint;
-    if (k < 0 || k >= K || __ldg(off + k) > w) k = 0;
-    int64_t step = 1;
-    while (k + step < K && __ldg(off + k + step) <= w) {
-        k += step;
-        step <<= 1;
-    }
-    int64_t hi = (k + step < K) ? k + step : K;
-    while (hi - k > 1) {
-        const int64_t mid = (k + hi) >> 1;
-        if (__ldg(off + mid) <= w) k = mid; else hi = mid;
-    }
-    return k;
-}
-
-template <int BOUND, bool EXACT>
-__device__ __forceinline__ float bound_at(const TrialRow &r, float ixf, int ix,
-                                          const SingleParams &p, int64_t k) {
-    if (BOUND == SSM_BOUND_CONSTANT) {
-        return r.a;
-    } else if (BOUND == SSM_BOUND_LINEAR) {
-        // table value a + f32(ix*dt) * p1 (boundary_functions.py:57-72 on t_s)
-        if (EXACT) return __fadd_rn(r.a, __fmul_rn(__fmul_rn(ixf, p.dt), r.p1));
-        return fmaf(ixf, r.dtp1, r.a);
-    } else if (BOUND == SSM_BOUND_WEIBULL) {
-        // a * exp(-(t/beta)^alpha) (boundary_functions.py:103-122)
-        const float x = ixf * p.dt * r.inv_beta;
-        const float pw = (x > 0.f) ? exp2f(r.p1 * __log2f(x)) : 0.f;
-        return r.a * __expf(-pw);
-    } else {
-        const int64_t i = (ix < p.tlen) ? ix : p.tlen - 1;
-        return __ldg(p.table + k * p.tstride + i);
-    }
-}
-
-// sin x and cos x on [0, pi/2] from their Taylor series through x^11 and x^12
-// (truncation errors below 6e-8 and 7e-9 there): short branch-free code for
-// the stable sampler, whose angles are always reduced to that interval.
-__device__ __forceinline__ float sin_q(float x) {
-    const float t = x * x;
-    float p = fmaf(t, -2.5052108e-08f, 2.7557319e-06f);  // -1/11!, 1/9!
-    p = fmaf(t, p, -1.9841270e-04f);                     // -1/7!
-    p = fmaf(t, p, 8.3333333e-03f);                      // 1/5!
-    p = fmaf(t, p, -1.6666667e-01f);                     // -1/3!
-    p = fmaf(t, p, 1.0f);
-    return x * p;
-}
-__device__ __forceinline__ float cos_q(float x) {
-    const float t = x * x;
-    float p = fmaf(t, 2.0876757e-09f, -2.7557319e-07f);  // 1/12!, -1/10!
-    p = fmaf(t, p, 2.4801587e-05f);                      // 1/8!
-    p = fmaf(t, p, -1.3888889e-03f);                     // -1/6!
-    p = fmaf(t, p, 4.1666667e-02f);                      // 1/4!
-    p = fmaf(t, p, -0.5f);
-    return fmaf(t, p, 1.0f);
-}
-
-// Symmetric alpha-stable variate by Chambers-Mallows-Stuck (Chambers, Mallows
-// & Stuck, JASA 71, 1976) with the reference's guards (_utils.pyx:426-472):
-// U ~ U(-pi/2 + 1e-7, pi/2 - 1e-7), W ~ Exp(1) floored at 1e-10, output
-// clipped to +-1e10 and NaN -> 0.
-//   X = sin(alpha U) / cos(U)^(1/alpha) * (cos((1 - alpha) U) / W)^((1 - alpha) / alpha)
-// (tan U for alpha = 1).  U = pi (u - 1/2) with u on a 2^-23 grid; the sampler
-// works with |U| and its complement V = pi/2 - |U| = pi min(u, 1 - u), which
-// carries one rounding only, so cos U = sin V keeps its relative precision as
-// |U| -> pi/2, where the heavy tail comes from.  Both powers are taken as one
-// power of two.
-__device__ __forceinline__ float cms_stable(uint32_t bu, uint32_t bw, const TrialRow &r) {
-    const float u01 = bits_to_1_2(bu) - 1.0f;
-    const float m = fmaxf(0.5f - fabsf(u01 - 0.5f), 3.1830988e-08f);  // V >= 1e-7 (the U clamp)
-    const float V = 3.14159265f * m;
-    const float aU = 1.57079633f - V;  // |U|
-    const float W = fmaxf(-0.69314718f * lg2_ftz(uniform_open(bw)), 1e-10f);
-    float X;
-    if (r.alpha == 1.0f) {
-        X = cos_q(V) / sin_q(V);  // |tan U|
-    } else {
-        const float cu = sin_q(V);                                             // cos U > 0
-        // cos((1 - alpha) U) = cos(c |U|), c = |1 - alpha| <= 1, evaluated as
-        // sin(pi/2 - c |U|) = sin(pi/2 (1 - c) + c V): two non-negative terms,
-        // so the argument does not cancel, and one polynomial serves every c |U|
-        const float c = fabsf(1.0f - r.alpha);
-        const float cua = fmaxf(sin_q(fmaf(c, V, 1.57079633f * (1.0f - c))), 1e-10f);
-        // alpha |U| in [0, pi); past pi/2 use pi - alpha |U| = pi (1 - alpha/2) + alpha V,
-        // which does not cancel as alpha -> 2
-        float A = r.alpha * aU;
-        if (A > 1.57079633f) A = fmaf(r.alpha, V, 3.14159265f * fmaf(-0.5f, r.alpha, 1.0f));
-        const float e = fmaf(r.expo, lg2_ftz(cua) - lg2_ftz(W), -r.inv_alpha * lg2_ftz(cu));
-        float p2;
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p2) : "f"(e));
-        X = sin_q(A) * p2;  // |sin(alpha U)| ...
-    }
-    X = (u01 < 0.5f) ? -X : X;  // ... times sign(U): every factor but sin(alpha U) is even in U
-    if (X != X) X = 0.f;
-    return fminf(fmaxf(X, -1e10f), 1e10f);
-}
-
 // Euler steps per block.  The Gaussian models draw six increments per
 // Philox4x32-10 call (three Box-Muller pairs, see bm6_increment), so a
 // 36-step block makes six independent Philox calls whose latencies overlap.
@@ -281,20 +130,14 @@ __device__ __forceinline__ float cms_stable(uint32_t bu, uint32_t bw, const Tria
 // spilled).  With the draws fused into the steps (step_block FUSE) 36 steps
 // fit for the constant and linear bounds (11.42 -> 11.00 ms against 24); the
 // Weibull and table bounds keep 24 (at 36 the Weibull bound spills 294 bytes).
-// The Levy model keeps 8-step blocks (its stable draws already give each
-// block enough independent work; 16-step blocks measured 8 % slower there).
+// The Levy model takes 16-step blocks: 512 sets of 10 000, 15.4 ms against 15.8
+// for 8 steps, 16.3 for 24 and 17.1 for 32 (which spill).
 // Call h of block b uses counter (BLK/6) b + h, so a stream does not depend
 // on the block length.
 template <int MODEL, int BOUND = SSM_BOUND_CONSTANT> struct Blk {
     static constexpr int value =
-        (MODEL == M_LEVY) ? 8
+        (MODEL == M_LEVY) ? 16
                           : ((MODEL == M_DFLEX && BOUND != SSM_BOUND_CONSTANT && BOUND != SSM_BOUND_LINEAR) ? 24 : 36);
-};
-// Lanes per walk W (see wide_block): 1 is the throughput mode above; W = 2,
-// 4, 8 give each trajectory an aligned group of W lanes and blocks of 18 W
-// steps, three Philox calls per lane.
-template <int MODEL, int W, int BOUND = SSM_BOUND_CONSTANT> struct BlkW {
-    static constexpr int value = (W == 1) ? Blk<MODEL, BOUND>::value : 18 * W;
 };
 // Device-RNG Gaussian models draw their increments inside the step loop
 // (step_block FUSE).  Outputs are bit-identical to drawing the block first;
@@ -304,40 +147,29 @@ template <int MODEL, int W, int BOUND = SSM_BOUND_CONSTANT> struct BlkW {
 template <int MODEL, bool NOISE> struct FuseOk {
     static constexpr bool value = !NOISE && MODEL != M_LEVY;
 };
-template <int MODEL, bool NOISE, int BOUND> struct WideOk {
-    static constexpr bool value =
-        !NOISE && MODEL != M_LEVY && MODEL != M_DFLEX && BOUND != SSM_BOUND_TABLE;
-};
-// Resident 256-thread CTAs per SM the compiler must fit (register cap
-// 65536 / (256 n)): 3 (80 registers) for blocks longer than 8 steps, 4 otherwise
-// (and 4 for the lanes-per-walk mode, whose lanes hold 18 increments).
-template <int MODEL, int W = 1> struct MinCtas {
-    static constexpr int value = (W == 1 && Blk<MODEL>::value > 8) ? 3 : 4;
-};
+// Increments drawn together: two Philox calls' twelve, whose Box-Muller pairs
+// share packed instructions (4 096-set angle batch 25.4 -> 24.4 ms against one
+// call's six at a time); one call's six for a Weibull bound, whose own arithmetic
+// needs the registers (256 sets: 4.41 ms against 4.67 with twelve).
+template <int BOUND> struct DrawN { static constexpr int value = (BOUND == SSM_BOUND_WEIBULL) ? 6 : 12; };
 
-struct Lane {
-    int64_t w;
-    uint32_t k, n, blk;
-    int ix;           // steps taken (maintained where an integer index is needed)
-    float y, tp, ixf; // position, float32 time accumulator, steps taken as float (see step_block)
-    float tpb;        // time accumulator at the start of the current block
-    float dinc;       // SDV/FULL: this trajectory's drift increment (v + sv g) dt
-};
-
-// models whose drift is drawn once per trajectory
-template <int MODEL> struct DrawnDrift { static constexpr bool value = (MODEL == M_SDV || MODEL == M_FULL); };
-
-// Increments 6h .. 6h+5 of the lane's current block from the device RNG
-// (Gaussian models): Philox call (BLK/6) blk + h of the trajectory's stream.
+// Increments DrawN h .. DrawN (h + 1) - 1 of the lane's current block from the
+// device RNG (Gaussian models): Philox calls (BLK/6) blk + ... of the
+// trajectory's stream, six increments each.
 template <int MODEL, int BOUND>
-__device__ __forceinline__ void draw_call(const SingleParams &p, const Lane &L, const TrialRow &r, int h,
-                                          float *g6) {
-    constexpr int BLK = Blk<MODEL, BOUND>::value;
+__device__ __forceinline__ void draw_calls(const SingleParams &p, const Lane &L, const TrialRow &r, int h,
+                                           float *g) {
+    constexpr int BLK = Blk<MODEL, BOUND>::value, C = DrawN<BOUND>::value / 6;
     // ddm_flex: drift 0 here, v(t_ix) dt from the table in the step
     const float drift = (MODEL == M_DFLEX) ? 0.f : (DrawnDrift<MODEL>::value ? L.dinc : r.drift);
-    const uint4 b = philox10(make_uint4((uint32_t)(BLK / 6) * L.blk + (uint32_t)h, L.n, L.k + p.k_base, 0u),
-                             p.key);
-    bm6_increment(b, r.c2, drift, g6);
+    const uint32_t ctr = (uint32_t)(BLK / 6) * L.blk + (uint32_t)(C * h);
+    const uint4 b0 = philox10(make_uint4(ctr, L.n, L.k + p.k_base, 0u), p.key);
+    if constexpr (C == 1) {
+        bm6_increment(b0, r.c2, drift, g);
+    } else {
+        const uint4 b1 = philox10(make_uint4(ctr + 1u, L.n, L.k + p.k_base, 0u), p.key);
+        bm12_increment(b0, b1, r.c2, drift, g);
+    }
 }
 
 // The block's increments.  Noise injection returns the raw caller draws (the
@@ -354,19 +186,21 @@ __device__ __forceinline__ void draw_block(const SingleParams &p, const Lane &L,
 #pragma unroll
         for (int q = 0; q < BLK; ++q) g[q] = (L.ix + OFF + q < p.nlen) ? __ldg(row + L.ix + q) : 0.f;
     } else if (MODEL == M_LEVY) {
+        // two variates per call; calls count in groups of four (eight steps), whatever the block length
 #pragma unroll
-        for (int h = 0; h < BLK / 2; h += 2) {
-            const uint4 b = philox10(make_uint4(L.blk, L.n, L.k + p.k_base, 2u + (uint32_t)h), p.key);
-            g[2 * h + 0] = fmaf(r.scale, cms_stable(b.x, b.y, r), r.drift);
-            g[2 * h + 1] = fmaf(r.scale, cms_stable(b.z, b.w, r), r.drift);
-            const uint4 c = philox10(make_uint4(L.blk, L.n, L.k + p.k_base, 3u + (uint32_t)h), p.key);
-            g[2 * h + 2] = fmaf(r.scale, cms_stable(c.x, c.y, r), r.drift);
-            g[2 * h + 3] = fmaf(r.scale, cms_stable(c.z, c.w, r), r.drift);
+        for (int h = 0; h < BLK / 2; ++h) {
+            const uint4 b = philox10(make_uint4((uint32_t)(BLK / 8) * L.blk + (uint32_t)(h / 4), L.n, L.k + p.k_base,
+                                                2u + (uint32_t)(h % 4)), p.key);
+            float x0, x1;
+            cms_stable2(b, r, x0, x1);
+            g[2 * h] = fmaf(r.scale, x0, r.drift);
+            g[2 * h + 1] = fmaf(r.scale, x1, r.drift);
         }
     } else {
-        static_assert(MODEL == M_LEVY || BLK % 6 == 0, "six increments per Philox call");
+        constexpr int DN = DrawN<BOUND>::value;
+        static_assert(MODEL == M_LEVY || BLK % DN == 0, "whole draws per block");
 #pragma unroll
-        for (int h = 0; h < BLK / 6; ++h) draw_call<MODEL, BOUND>(p, L, r, h, g + 6 * h);
+        for (int h = 0; h < BLK / DN; ++h) draw_calls<MODEL, BOUND>(p, L, r, h, g + DN * h);
     }
 }
 
@@ -383,7 +217,8 @@ __device__ __forceinline__ bool step_block(const SingleParams &p, Lane &L, const
                                            const float *g) {
     constexpr int BLK = Blk<MODEL, BOUND>::value;
     static_assert(!FUSE || (!NOISE && MODEL != M_LEVY), "fused draws: device RNG, Gaussian models");
-    float g6[6];
+    constexpr int DN = DrawN<BOUND>::value;
+    float gd[DN];
     if (L.ixf >= r.capf) {
         raise_error(p.hdr, SSM_ERR_DEVICE, (int)L.w);
         return false;
@@ -394,7 +229,12 @@ __device__ __forceinline__ bool step_block(const SingleParams &p, Lane &L, const
     // the linear bound is a + ixf0 slope dt plus q slope dt, and finalize()
     // recovers the steps of the last block from the time accumulator.
     const float ixf0 = L.ixf;
-    const float b0 = (!INT_IX && BOUND == SSM_BOUND_LINEAR) ? fmaf(ixf0, r.dtp1, r.a) : 0.f;
+    // (Levy: bases every eight steps)
+    constexpr int BB = (MODEL == M_LEVY) ? 8 : BLK;
+    float base[BLK / BB];
+#pragma unroll
+    for (int u = 0; u < BLK / BB; ++u)
+        base[u] = (!INT_IX && BOUND == SSM_BOUND_LINEAR) ? fmaf(ixf0 + (float)(BB * u), r.dtp1, r.a) : 0.f;
     if (!INT_IX) L.tpb = L.tp;
     const float *drow = (MODEL == M_DFLEX) ? p.dtable + (int64_t)L.k * p.dstride : nullptr;
     // device RNG: the block's drifts v(t_ix .. t_ix+BLK-1) are read before
@@ -418,8 +258,8 @@ __device__ __forceinline__ bool step_block(const SingleParams &p, Lane &L, const
     bool live = true;
 #pragma unroll
     for (int q = 0; q < BLK; ++q) {
-        if (FUSE && q % 6 == 0) draw_call<MODEL, BOUND>(p, L, r, q / 6, g6);
-        const float gq = FUSE ? g6[q % 6] : g[q];
+        if (FUSE && q % DN == 0) draw_calls<MODEL, BOUND>(p, L, r, q / DN, gd);
+        const float gq = FUSE ? gd[q % DN] : g[q];
         bool inside;
         // the time test; a block whose every step is known to pass it skips it (TCHK false)
         const bool in_time = !TCHK || (L.tp <= r.dl_tmp);
@@ -428,7 +268,7 @@ __device__ __forceinline__ bool step_block(const SingleParams &p, Lane &L, const
         } else {
             float b;
             if (INT_IX) b = bound_at<BOUND, NOISE>(r, L.ixf, L.ix, p, L.k);
-            else if (BOUND == SSM_BOUND_LINEAR) b = (q == 0) ? b0 : fmaf((float)q, r.dtp1, b0);
+            else if (BOUND == SSM_BOUND_LINEAR) b = (q % BB == 0) ? base[q / BB] : fmaf((float)(q % BB), r.dtp1, base[q / BB]);
             else b = bound_at<BOUND, NOISE>(r, ixf0 + (float)q, 0, p, L.k);
             inside = live && (fabsf(L.y) <= b) && in_time;
         }
@@ -477,21 +317,20 @@ __device__ __forceinline__ bool step_block(const SingleParams &p, Lane &L, const
 // additions' rounding; below 65536 dt an ulp of t is at most dt/64, so that
 // rounding stays under dt/4, and t + (BLK+1) dt <= dl_tmp, evaluated in float,
 // leaves more than that margin.
-template <int MODEL, int BOUND, bool NOISE, int BLK = Blk<MODEL, BOUND>::value>
+template <int MODEL, int BOUND, bool NOISE>
 __device__ __forceinline__ bool block_in_time(const SingleParams &p, const Lane &L, const TrialRow &r) {
     constexpr bool INT_IX = NOISE || BOUND == SSM_BOUND_TABLE;
     if (INT_IX) return false;
-    // longer blocks (lanes-per-walk mode, 36-144 steps) keep a margin of
-    // 2 dt per 64 steps: past 65536 dt an addition rounds by up to dt/64
-    constexpr float SPAN = (float)(BLK + 1 + 2 * (BLK / 64));
+    constexpr float SPAN = (float)(Blk<MODEL, BOUND>::value + 1);
     return (L.tp < p.dt * 65536.f) && (fmaf(SPAN, p.dt, L.tp) <= r.dl_tmp);
 }
 
 // Steps taken by a walk that has ended.  Without an integer index L.ixf
 // counts whole blocks; the steps of the last block are those that took the
 // time accumulator from L.tpb to L.tp (the same float additions replayed).
-template <int MODEL, int BOUND, bool NOISE, int BLK = Blk<MODEL, BOUND>::value>
+template <int MODEL, int BOUND, bool NOISE>
 __device__ __forceinline__ int steps_taken(const SingleParams &p, const Lane &L) {
+    constexpr int BLK = Blk<MODEL, BOUND>::value;
     constexpr bool INT_IX = NOISE || BOUND == SSM_BOUND_TABLE;
     if (INT_IX) return (int)L.ixf;
     float tt = L.tpb;
@@ -503,187 +342,47 @@ __device__ __forceinline__ int steps_taken(const SingleParams &p, const Lane &L)
     return (int)L.ixf - BLK + c;
 }
 
-template <int MODEL, int BOUND, bool NOISE, int BLK = Blk<MODEL, BOUND>::value>
-__device__ __forceinline__ void finalize(const SingleParams &p, const Lane &L, bool writer = true) {
-    // fields needed only here are re-read instead of being held across the walk
-    const TrialRow *row = p.rows + L.k;
-    const float t = __ldg(&row->t), deadline = __ldg(&row->deadline), dl = __ldg(&row->dl_tmp);
-    float u;
-    if (NOISE) u = __ldg(p.nunif + L.w * p.ustride + (p.ustride - 1));
-    else u = uniform_co(philox10(make_uint4(0u, L.n, L.k + p.k_base, 1u), p.key).x);
-    float tt = t;
-    if (MODEL == M_FULL) {
-        // t + 2 (u - 0.5) st in double (ddm_models.pyx:2253); the same uniform as at the start
-        float ut;
-        if (NOISE) ut = __ldg(p.nunif + L.w * p.ustride);
-        else ut = uniform_co(philox10(make_uint4(0u, L.n, L.k + p.k_base, 3u), p.key).z);
-        tt = __double2float_rn((double)t + (2.0 * ((double)ut - 0.5)) * (double)__ldg(&row->expo));
-    }
-    // compute_smooth_unif (_utils.pyx:668-695): double arithmetic, float result
-    float sm = 0.f;
-    if (p.smooth) {
-        if (L.tp == 0.f) sm = __double2float_rn(((double)u * 0.5) * (double)p.dt);
-        else if (L.tp < dl) sm = __double2float_rn((0.5 - (double)u) * (double)p.dt);
-    }
-    float rt = __fadd_rn(__fadd_rn(L.tp, tt), sm);
-    if (rt >= deadline || deadline <= 0.f) rt = -999.f;  // enforce_deadline
-    const int choice = (L.y > 0.f) - (L.y < 0.f);         // sign(y)
-    if (!writer) return;
-    p.rts[L.w] = rt;
-    p.choices[L.w] = choice;
-    if (p.steps) p.steps[L.w] = steps_taken<MODEL, BOUND, NOISE, BLK>(p, L);
-}
-
-// Start lane L on the trajectory with queue index w; false (and the error
-// word set) if a caller-given processing order does not cover that index.
-template <int MODEL, bool NOISE>
-__device__ __forceinline__ bool lane_init(const SingleParams &p, Lane &L, TrialRow &r, int64_t w,
-                                          int64_t &hint) {
-    int64_t k, n;
-    if (p.offsets == nullptr) {
-        k = w % p.n_trials;
-        n = w / p.n_trials;
-    } else if (p.order != nullptr) {
-        // queue index -> position j in the processing order -> trial k; the
-        // output index stays offsets[k] + n, so results do not depend on the order
-        const int64_t j = ragged_find(p.qoff, p.n_trials, w, hint);
-        hint = j;
-        k = __ldg(p.order + j);
-        n = w - __ldg(p.qoff + j);
-        if (k < 0 || k >= p.n_trials || n < 0 || n >= __ldg(p.offsets + k + 1) - __ldg(p.offsets + k)) {
-            raise_error(p.hdr, SSM_ERR_ARG, (int)j);
-            return false;
-        }
-        w = __ldg(p.offsets + k) + n;
-    } else {
-        w += __ldg(p.offsets);  // global output index (trial windows start past 0)
-        k = ragged_find(p.offsets, p.n_trials, w, hint);
-        n = w - __ldg(p.offsets + k);
-        hint = k;
-    }
-    const float4 *src = reinterpret_cast<const float4 *>(p.rows + k);
-    float4 *dst = reinterpret_cast<float4 *>(&r);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dst[i] = __ldg(src + i);
-    L.w = w;
-    L.k = (uint32_t)k;
-    L.n = (uint32_t)n;
-    L.blk = 0;
-    L.ix = 0;
-    L.ixf = 0.f;
-    L.tp = 0.f;
-    L.y = r.y0;
-    if (DrawnDrift<MODEL>::value) {
-        // per-trajectory drift normal and (full_ddm) start-point uniform
-        // (ddm_models.pyx:2249-2266): injected, or drawn from the trajectory's stream
-        float g0, uy = 0.5f;
-        if (NOISE) {
-            g0 = __ldg(p.noise + L.w * p.nlen);
-            if (MODEL == M_FULL) uy = __ldg(p.nunif + L.w * p.ustride + 1);
-        } else {
-            const uint4 b = philox10(make_uint4(0u, L.n, L.k + p.k_base, 3u), p.key);
-            g0 = box_muller(b.x, b.y).x;
-            uy = uniform_co(b.w);
-        }
-        L.dinc = __fmul_rn(__fadd_rn(r.drift, __fmul_rn(r.alpha, g0)), p.dt);
-        if (MODEL == M_FULL)
-            L.y = __double2float_rn((double)L.y + (2.0 * ((double)uy - 0.5)) * (double)r.inv_alpha);
-    }
-    return true;
-}
-
-// One block of the lanes-per-walk mode (W = 2, 4, 8; device RNG, in-register
-// boundaries).  The W lanes of an aligned group carry one trajectory and
-// hold identical state.  A block is 18 W steps: lane s of the group makes
-// Philox calls 3 W b + 3 s + m (m = 0, 1, 2) of block b -- the counters the
-// one-lane mode uses for the same steps -- and every lane of the group then
-// runs the block's steps in order, each increment broadcast by a shuffle from
-// the lane that drew it.  The warp issues about 8 instructions per step of
-// 32 / W walks instead of about 21 per step of 32: throughput traded for the
-// latency of one walk, which is what bounds a launch with fewer
-// trajectories than resident lanes.  18 W is a multiple of 36, so the linear
-// boundary comes from the same 36-step bases as in the one-lane mode and the
-// results are bit-identical to it.  Every lane of the warp takes part (the
-// shuffles need the whole warp); a lane without a running walk (`active`
-// false, possibly still holding an ended walk's state for finalize) changes
-// nothing.
-template <int MODEL, int BOUND, bool TCHK, int W>
-__device__ __forceinline__ bool wide_block(const SingleParams &p, Lane &L, const TrialRow &r, bool active,
-                                           int src0, int sub) {
-    static_assert(W == 2 || W == 4 || W == 8, "lanes per walk");
-    constexpr int BLK = 18 * W;
-    constexpr unsigned FULL = 0xffffffffu;
-    const bool capped = active && L.ixf >= r.capf;
-    if (capped) raise_error(p.hdr, SSM_ERR_DEVICE, (int)L.w);
-    bool live = active && !capped;
-    const float drift = DrawnDrift<MODEL>::value ? L.dinc : r.drift;
-    float g[18];
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-        const uint4 b = philox10(
-            make_uint4((uint32_t)(3 * W) * L.blk + (uint32_t)(3 * sub + m), L.n, L.k + p.k_base, 0u), p.key);
-        bm6_increment(b, r.c2, drift, g + 6 * m);
-    }
-    const float ixf0 = L.ixf;
-    float b36[W / 2];  // linear boundary at the block's 36-step bases
-#pragma unroll
-    for (int u = 0; u < W / 2; ++u)
-        b36[u] = (BOUND == SSM_BOUND_LINEAR) ? fmaf(ixf0 + (float)(36 * u), r.dtp1, r.a) : 0.f;
-    if (live) L.tpb = L.tp;
-#pragma unroll
-    for (int s = 0; s < W; ++s) {
-#pragma unroll
-        for (int j = 0; j < 18; ++j) {
-            const float gq = __shfl_sync(FULL, g[j], src0 + s);
-            const int q = 18 * s + j;
-            const bool in_time = !TCHK || (L.tp <= r.dl_tmp);
-            bool inside;
-            if (MODEL == M_LEGACY) {
-                inside = live && (L.y <= r.a) && (L.y >= 0.f) && in_time;
-            } else {
-                float bq;
-                if (BOUND == SSM_BOUND_LINEAR)
-                    bq = (q % 36 == 0) ? b36[q / 36] : fmaf((float)(q % 36), r.dtp1, b36[q / 36]);
-                else
-                    bq = bound_at<BOUND, false>(r, ixf0 + (float)q, 0, p, L.k);
-                inside = live && (fabsf(L.y) <= bq) && in_time;
-            }
-            if (inside) {
-                if (MODEL == M_OU) L.y = fmaf(L.y, r.expo, gq);
-                else L.y += gq;
-                L.tp += p.dt;
-            }
-            live = inside;
-        }
-    }
-    if (active && !capped) L.ixf = ixf0 + (float)BLK;
-    return live;
+// Write an ended walk's outputs.  With LATE the time is written as it is and
+// k_finish turns the whole array into rts: a warp finishes few walks at a time,
+// so the jitter's Philox call and the rest of finish_rt would run here with
+// most lanes idle (about 100 instructions per pass, 5 % of the launch).
+template <int MODEL, int BOUND, bool NOISE, bool LATE>
+__device__ __forceinline__ void finalize(const SingleParams &p, const Lane &L) {
+    p.rts[L.w] = LATE ? L.tp : finish_rt<MODEL, NOISE>(p, L.k, L.n, L.w, L.tp);
+    p.choices[L.w] = (L.y > 0.f) - (L.y < 0.f);  // sign(y)
+    if (p.steps) p.steps[L.w] = steps_taken<MODEL, BOUND, NOISE>(p, L);
 }
 
 // ------------------------------------------------------------------ main kernel
-// W lanes per walk (1 = one lane per trajectory; 2, 4, 8 = wide_block).  The
-// queue logic counts walks: a group's lanes share `active`, so a ballot of
-// free lanes holds W bits per free walk.
-template <int MODEL, int BOUND, bool NOISE, int W>
-__global__ void __launch_bounds__(256, (MinCtas<MODEL, W>::value))
-    k_single(const __grid_constant__ SingleParams p) {
-    static_assert(W == 1 || WideOk<MODEL, NOISE, BOUND>::value, "lanes per walk > 1: device RNG, in-register bound");
-    constexpr int BLK = BlkW<MODEL, W, BOUND>::value;
+// One lane per walk.  80 registers: three 256-thread CTAs per SM; more resident
+// warps measured no faster (24.4 ms with 24 to 32 warps per SM).
+template <int MODEL, int BOUND, bool NOISE>
+__global__ void __launch_bounds__(256, 3) k_single(const __grid_constant__ SingleParams p) {
+    constexpr int BLK = Blk<MODEL, BOUND>::value;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const int sub = lane & (W - 1);              // place in the group
-    const int src0 = lane - sub;                 // the group's first lane
-    const unsigned lt_mask = (1u << src0) - 1u;  // lanes of the groups before this one
+    const unsigned lt_mask = (1u << lane) - 1u;
     const int64_t total = (p.total >= 0) ? p.total : __ldg(p.offsets + p.n_trials) - __ldg(p.offsets);
-    const int64_t chunk = warp_chunk(p.chunk, total, 32 / W);
+    const int64_t chunk = warp_chunk(p.chunk, total);
 
     Lane L;
     TrialRow r = {};
-    L.w = 0; L.k = L.n = L.blk = 0; L.ix = 0; L.y = L.tp = L.ixf = L.dinc = L.tpb = 0.f;
+    L.w = 0; L.k = NO_TRIAL; L.n = L.blk = 0; L.ix = 0; L.y = L.tp = L.ixf = L.dinc = L.tpb = 0.f;
     bool active = false;
     bool pending = false;  // walk ended, result not yet written
     bool exhausted = false;
     int64_t q_next = 0, q_end = 0, hint = 0;
+    // The last trial this warp looked up (the same in every lane).  A claim is
+    // consecutive queue indices, so most restarts stay in it: the next `left` of
+    // them are its samples n_next, n_next + 1, ... with outputs from w_next, and need
+    // neither the queue nor a search (q_next is brought up to date by left0 -
+    // left when they run out).
+    Span sp = {0, 0, 0, 0u};
+    if (p.offsets == nullptr && p.n_trials == 1) sp.hi = total;
+    int64_t w_next = 0;
+    uint32_t n_next = 0u;
+    int left = 0, left0 = 0;
+    constexpr bool LATE = !NOISE;  // rts by k_finish (see finalize)
 
     for (;;) {
         // Lanes whose walk ended wait (predicated off) until refill_min of
@@ -691,53 +390,106 @@ __global__ void __launch_bounds__(256, (MinCtas<MODEL, W>::value))
         // rest of the warp idle, so it is done for several lanes in one pass.
         // Once the queue is empty, pending results are written at once.
         const unsigned need = __ballot_sync(FULL, !active);
-        const int free_walks = __popc(need) / W;
-        const bool pass = exhausted ? (__ballot_sync(FULL, pending) != 0u) : (free_walks >= p.refill_min);
-        if (pass && pending) {
-            finalize<MODEL, BOUND, NOISE, BLK>(p, L, sub == 0);
-            pending = false;
-        }
-        if (pass && !exhausted) {
-            const int cnt = free_walks;
-            const int64_t avail = q_end - q_next;
-            int64_t base = 0;
-            if (avail < cnt) {
-                unsigned long long b = 0ull;
-                if (lane == 0) b = atomicAdd(&p.hdr->counter, (unsigned long long)chunk);
-                base = (int64_t)__shfl_sync(FULL, b, 0);
-                if (base >= total) exhausted = true;
+        const int cnt = __popc(need);
+        if (need != 0u && (exhausted || cnt >= p.refill_min)) {
+            if (pending) {
+                finalize<MODEL, BOUND, NOISE, LATE>(p, L);
+                pending = false;
             }
-            if (!active) {
-                const int rank = __popc(need & lt_mask) / W;
+            const int rank = __popc(need & lt_mask);
+            if (cnt <= left) {
+                if (!active) {
+                    lane_start<MODEL, NOISE>(p, L, r, w_next + rank, sp.k, n_next + (uint32_t)rank);
+                    active = true;
+                }
+                w_next += cnt;
+                n_next += (uint32_t)cnt;
+                left -= cnt;
+            } else if (!exhausted) {
+                q_next += left0 - left;
+                const int64_t avail = q_end - q_next;
+                int64_t base = 0;
+                if (avail < cnt) {
+                    unsigned long long b = 0ull;
+                    if (lane == 0) b = atomicAdd(&p.hdr->counter, (unsigned long long)chunk);
+                    base = (int64_t)__shfl_sync(FULL, b, 0);
+                    if ((uint64_t)base >= (uint64_t)total) exhausted = true;
+                }
                 const int64_t w = (rank < avail) ? q_next + rank : base + (rank - avail);
-                if (w < total) active = lane_init<MODEL, NOISE>(p, L, r, w, hint);
+                const bool start = !active && w < total;
+                if (p.offsets == nullptr) {
+                    if (start) {
+                        uint32_t k, n;
+                        layout_trial(p, w, k, n);
+                        lane_start<MODEL, NOISE>(p, L, r, w, k, n);
+                        active = true;
+                    }
+                } else {
+                    // the last restart's trial, searched by the whole warp, is the
+                    // next ones' most likely one; a restart of another trial
+                    // searches on its own
+                    const unsigned misses = __ballot_sync(FULL, start && !(w >= sp.lo && w < sp.hi));
+                    if (misses != 0u) {
+                        const int64_t last = __shfl_sync(FULL, w, 31 - __clz(misses));
+                        if (!find_span(p, last, hint, sp)) sp.lo = sp.hi = 0;
+                    }
+                    if (start) {
+                        Span mine = sp;
+                        int64_t from = hint;
+                        if ((w >= sp.lo && w < sp.hi) || find_span(p, w, from, mine)) {
+                            const int64_t n = w - mine.lo;
+                            lane_start<MODEL, NOISE>(p, L, r, mine.out0 + n, mine.k, (uint32_t)n);
+                            active = true;
+                        }
+                    }
+                    __syncwarp();
+                }
+                if (avail >= cnt) {
+                    q_next += cnt;
+                } else {
+                    q_next = base + (cnt - avail);
+                    q_end = base + chunk;
+                }
+                const int64_t in_span = (q_next >= sp.lo) ? sp.hi - q_next : 0;
+                left = left0 = exhausted ? 0 : (int)max(min(min(q_end, total) - q_next, in_span), (int64_t)0);
+                w_next = sp.out0 + (q_next - sp.lo);
+                n_next = (uint32_t)(q_next - sp.lo);
             }
-            if (avail >= cnt) {
-                q_next += cnt;
-            } else {
-                q_next = base + (cnt - avail);
-                q_end = base + chunk;
+        }
+        // (The exit test below stays outside the branch above: with the break inside
+        // it, one of the noise-injection kernels took the claim's shuffled base from
+        // the register of `need` -- found on bounded, index-checked copies.)
+        // The queue is empty and few of the warp's walks still run: a walk here
+        // takes the time of a whole warp's steps, a walk with eight lanes of its
+        // own a tenth of it, so they are left to the lanes-per-walk kernel.
+        if (p.left != nullptr && exhausted) {
+            const unsigned on = __ballot_sync(FULL, active);
+            if (__popc(on) <= LEAVE_MAX) {
+                unsigned long long b = 0ull;
+                if (lane == 0) b = atomicAdd(&p.hdr->aux[0], (unsigned long long)__popc(on));
+                b = __shfl_sync(FULL, b, 0);
+                if (active) {
+                    LeftWalk &o = p.left[b + __popc(on & lt_mask)];
+                    o.w = L.w; o.k = L.k; o.n = L.n;
+                    o.y = L.y; o.tp = L.tp; o.ixf = L.ixf; o.dinc = L.dinc;
+                    active = false;
+                }
             }
         }
         if (__ballot_sync(FULL, active) == 0u) break;
         // warp-uniform: skip the per-step time test when no active lane can reach its limit in this block
-        const bool skip_time = __all_sync(FULL, !active || block_in_time<MODEL, BOUND, NOISE, BLK>(p, L, r));
+        const bool skip_time = __all_sync(FULL, !active || block_in_time<MODEL, BOUND, NOISE>(p, L, r));
         bool live = false;
-        if constexpr (W == 1) {
-            if (active) {
-                if constexpr (FuseOk<MODEL, NOISE>::value) {
-                    live = skip_time ? step_block<MODEL, BOUND, NOISE, false, false, true>(p, L, r, nullptr)
-                                     : step_block<MODEL, BOUND, NOISE, false, true, true>(p, L, r, nullptr);
-                } else {
-                    float g[Blk<MODEL, BOUND>::value];
-                    draw_block<MODEL, BOUND, NOISE>(p, L, r, g);
-                    live = skip_time ? step_block<MODEL, BOUND, NOISE, false, false>(p, L, r, g)
-                                     : step_block<MODEL, BOUND, NOISE, false, true>(p, L, r, g);
-                }
+        if (active) {
+            if constexpr (FuseOk<MODEL, NOISE>::value) {
+                live = skip_time ? step_block<MODEL, BOUND, NOISE, false, false, true>(p, L, r, nullptr)
+                                 : step_block<MODEL, BOUND, NOISE, false, true, true>(p, L, r, nullptr);
+            } else {
+                float g[BLK];
+                draw_block<MODEL, BOUND, NOISE>(p, L, r, g);
+                live = skip_time ? step_block<MODEL, BOUND, NOISE, false, false>(p, L, r, g)
+                                 : step_block<MODEL, BOUND, NOISE, false, true>(p, L, r, g);
             }
-        } else {
-            live = skip_time ? wide_block<MODEL, BOUND, false, W>(p, L, r, active, src0, sub)
-                             : wide_block<MODEL, BOUND, true, W>(p, L, r, active, src0, sub);
         }
         if (active) {
             L.blk += 1;
@@ -745,6 +497,32 @@ __global__ void __launch_bounds__(256, (MinCtas<MODEL, W>::value))
                 active = false;
                 pending = true;
             }
+        }
+    }
+}
+
+// The rts of a launch whose walks wrote their bare times (finalize LATE): one
+// thread per output, full warps.  Each CTA takes runs of FINISH_RUN consecutive
+// outputs, so one search places the run and the threads walk on from there.
+constexpr int FINISH_RUN = 2048;
+template <int MODEL>
+__global__ void __launch_bounds__(256) k_finish(const __grid_constant__ SingleParams p) {
+    const int64_t w0 = p.offsets ? __ldg(p.offsets) : 0;
+    const int64_t total = (p.total >= 0) ? p.total : __ldg(p.offsets + p.n_trials) - w0;
+    for (int64_t b = (int64_t)blockIdx.x * FINISH_RUN; b < total; b += (int64_t)gridDim.x * FINISH_RUN) {
+        int64_t hint = 0;
+#pragma unroll 2
+        for (int64_t i = b + threadIdx.x; i < min(b + FINISH_RUN, total); i += 256) {
+            uint32_t k, n;
+            if (p.offsets == nullptr) {
+                layout_trial(p, i, k, n);
+            } else {
+                hint = ragged_find(p.offsets, p.n_trials, w0 + i, hint);
+                k = (uint32_t)hint;
+                n = (uint32_t)(w0 + i - __ldg(p.offsets + hint));
+            }
+            const float tp = p.rts[w0 + i];
+            p.rts[w0 + i] = finish_rt<MODEL, false>(p, k, n, w0 + i, tp);
         }
     }
 }
@@ -758,8 +536,11 @@ __global__ void k_record(const __grid_constant__ SingleParams p) {
     if (threadIdx.x != 0) return;
     Lane L;
     TrialRow r;
-    int64_t hint = 0;
-    lane_init<MODEL, NOISE>(p, L, r, 0, hint);
+    // sample 0 of the first trial that has one
+    L.k = NO_TRIAL;
+    int64_t k0 = 0;
+    if (p.offsets != nullptr) k0 = ragged_find(p.offsets, p.n_trials, __ldg(p.offsets), 0);
+    lane_start<MODEL, NOISE>(p, L, r, p.offsets ? __ldg(p.offsets + k0) : 0, (uint32_t)k0, 0u);
     if (p.traj_len > 0) p.traj[0] = L.y;
     for (;;) {
         float g[Blk<MODEL, BOUND>::value];
@@ -783,52 +564,63 @@ int auto_lanes_per_walk(int64_t n_walks) {
     return 1;
 }
 
-struct Launcher {
-    template <int MODEL, int BOUND, bool NOISE, int W>
-    static int launch(const SingleParams &p, int threads, const ssm_launch *opt, cudaStream_t st) {
-        auto kern = k_single<MODEL, BOUND, NOISE, W>;
-        int per_sm = 0;
-        SSM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0));
-        if (opt && opt->blocks_per_sm > 0 && opt->blocks_per_sm < per_sm) per_sm = opt->blocks_per_sm;
-        if (per_sm < 1) per_sm = 1;
-        kern<<<sm_count() * per_sm, threads, 0, st>>>(p);
-        SSM_CUDA(cudaGetLastError());
-        return SSM_OK;
+// The lanes a launch really takes.  Asked for 8, a launch of known size takes wider
+// groups as long as the GPU holds them; asked for 2 or 4 it runs one lane per
+// walk and hands its last walks over (left: it has the room for them), which has
+// overtaken both.  Plain DDM, one parameter set, us for 1 / 4 / 8 / 16 / 32 lanes
+// (one lane without and with handing over): 1 000 walks 266, 160 / 120 / 78 / 57 /
+// 47; 10 000 385, 215 / 175 / 120 / 92 / 106; 30 000 407, 256 / 219 / 161 / 170 /
+// 243; 100 000 613, 353 / 360 / 351 / 445 / 721; 300 000 778, 549 / 749 / 904.
+static int effective_lanes(int W, int64_t total, bool left) {
+    const int64_t warps = (int64_t)sm_count() * 24;
+    if (total >= 0) {
+        if (W < 8) return (W == 4 && (!left || total <= 24 * warps)) ? 8 : 1;
+        return (total <= warps) ? 32 : (total <= 4 * warps) ? 16 : 8;
     }
+    return (W == 8 || (W == 4 && !left)) ? 8 : 1;
+}
 
+struct Launcher {
     template <int MODEL, int BOUND, bool NOISE>
-    static int run(const SingleParams &p, const ssm_launch *opt, cudaStream_t st) {
+    static int run(const SingleParams &call, const ssm_launch *opt, cudaStream_t st) {
         int threads = (opt && opt->block_threads > 0) ? opt->block_threads : 256;
         if (threads > 256 || threads % 32) {
             set_error("block_threads must be a multiple of 32 and at most 256");
             return SSM_ERR_ARG;
         }
         constexpr bool WIDE = WideOk<MODEL, NOISE, BOUND>::value;
-        const int W = (opt && opt->lanes_per_walk > 0) ? opt->lanes_per_walk
-                                                        : (WIDE && p.total >= 0 ? auto_lanes_per_walk(p.total) : 1);
-        if (W != 1 && W != 2 && W != 4 && W != 8) {
-            set_error("lanes_per_walk must be 0 (automatic), 1, 2, 4 or 8");
+        int W = (opt && opt->lanes_per_walk > 0) ? opt->lanes_per_walk : 1;
+        if (W != 1 && W != 2 && W != 4 && W != 8 && W != 16 && W != 32) {
+            set_error("lanes_per_walk must be 0 (automatic), 1, 2, 4, 8, 16 or 32");
             return SSM_ERR_ARG;
         }
         if (W > 1 && !WIDE) {
             set_error("lanes_per_walk > 1 needs the device RNG and a constant, linear or Weibull boundary");
             return SSM_ERR_ARG;
         }
-        int rc = SSM_OK;
-        if (W == 1) {
-            rc = launch<MODEL, BOUND, NOISE, 1>(p, threads, opt, st);
-        } else if constexpr (WIDE) {
-            // a warp holds 32 / W walks: it claims that many at a time and
-            // restarts a group as soon as its walk ends (unless told otherwise)
-            SingleParams q = p;
-            const int slots = 32 / W;
-            q.chunk = slots;
-            q.refill_min = (opt && opt->refill_min > 0) ? min(opt->refill_min, slots) : 1;
-            rc = (W == 2)   ? launch<MODEL, BOUND, NOISE, 2>(q, threads, opt, st)
-                 : (W == 4) ? launch<MODEL, BOUND, NOISE, 4>(q, threads, opt, st)
-                            : launch<MODEL, BOUND, NOISE, 8>(q, threads, opt, st);
+        if (WIDE && call.total >= 0 && !(opt && opt->lanes_per_walk > 0)) W = auto_lanes_per_walk(call.total);
+        if (WIDE && W > 1 && W <= 8) W = effective_lanes(W, call.total, call.left != nullptr);
+        if (W > 1) return wide_launch(MODEL, BOUND, W, call, opt, st);
+        SingleParams p = call;
+        if (NOISE || BOUND == SSM_BOUND_TABLE) p.left = nullptr;
+        auto kern = k_single<MODEL, BOUND, NOISE>;
+        int per_sm = 0;
+        SSM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0));
+        if (opt && opt->blocks_per_sm > 0 && opt->blocks_per_sm < per_sm) per_sm = opt->blocks_per_sm;
+        if (per_sm < 1) per_sm = 1;
+        kern<<<sm_count() * per_sm, threads, 0, st>>>(p);
+        SSM_CUDA(cudaGetLastError());
+        if (p.left != nullptr) {
+            const int rc = wide_finish(MODEL, BOUND, p, st);
+            if (rc != SSM_OK) return rc;
         }
-        if (rc != SSM_OK) return rc;
+        if (!NOISE) {
+            // up to 8 CTAs per SM; a known total needs no more than its runs
+            int64_t grid = (int64_t)sm_count() * 8;
+            if (p.total >= 0) grid = std::min(grid, (p.total + FINISH_RUN - 1) / FINISH_RUN);
+            k_finish<MODEL><<<(unsigned)grid, 256, 0, st>>>(p);
+            SSM_CUDA(cudaGetLastError());
+        }
         if (p.traj && p.traj_len > 0) {
             SingleParams pr = p;  // trial 0 / sample 0, whatever the processing order
             pr.order = nullptr;
@@ -866,10 +658,14 @@ struct Launcher {
     }
 };
 
+// The header and the rows are needed; with the room for the walks that the
+// one-lane kernel leaves (LEAVE_MAX for each of an SM's 64 warps) behind them the
+// launch hands its last walks over.
 static size_t single_ws_bytes(int64_t n_trials) {
     size_t b = sizeof(WorkspaceHeader) + (size_t)(n_trials > 0 ? n_trials : 0) * sizeof(TrialRow);
     return (b + 255) & ~(size_t)255;
 }
+static size_t left_bytes() { return (size_t)sm_count() * 64 * LEAVE_MAX * sizeof(LeftWalk); }
 
 struct SingleCall {
     int model;
@@ -968,6 +764,7 @@ static int run_single(const SingleCall &c) {
     p.noise = c.noise; p.nlen = c.nlen; p.nunif = c.nunif;
     p.rts = c.rts; p.choices = c.choices; p.steps = c.steps;
     p.hdr = hdr;
+    p.left = (c.ws_bytes >= need + left_bytes()) ? (LeftWalk *)((char *)c.ws + need) : nullptr;
     p.traj = c.traj; p.traj_len = c.traj_len;
     if (p.total == 0) {
         if (c.traj) {  // nothing simulated: trajectory metadata is all padding
@@ -991,7 +788,7 @@ static int run_single(const SingleCall &c) {
 
 extern "C" {
 
-size_t ssm_ddm_workspace_bytes(int64_t n_trials) { return ssm::single_ws_bytes(n_trials); }
+size_t ssm_ddm_workspace_bytes(int64_t n_trials) { return ssm::single_ws_bytes(n_trials) + ssm::left_bytes(); }
 int ssm_auto_lanes_per_walk(int64_t n_walks) { return ssm::auto_lanes_per_walk(n_walks); }
 
 int ssm_ddm_flexbound(const float *v, const float *a, const float *z, const float *t,
