@@ -2,15 +2,24 @@
 // (cssm.race_model, src/cssm/race_models.pyx:356-506) and the leaky competing
 // accumulator (cssm.lca, race_models.pyx:757-920).
 //
-// Same execution model as the single-accumulator kernel: one thread per
-// trajectory, persistent grid, warps refill finished lanes from a global work
-// counter.  The NP accumulators of a trajectory live in registers.  Each step
-// tests the reference's loop condition (no accumulator above b(t) and
+// One thread per trajectory, persistent grid, warps refill finished lanes from a
+// global work counter.  The NP accumulators of a trajectory live in registers.
+// Each step tests the reference's loop condition (no accumulator above b(t) and
 // t <= min(max_t, deadline - t_nd)), then updates every accumulator with its
 // own N(0,1) increment and clips it at 0.  Choices are argmax (first maximum).
-// Philox4x32-10 supplies four increments per call; noise injection reads
-// caller rows (draw index step * NP + j) and evaluates every float operation
-// with explicit rounding in the reference's order.
+// Noise injection reads caller rows (draw index step * NP + j) and evaluates
+// every float operation with explicit rounding in the reference's order.
+//
+// With the device RNG and up to four accumulators (k_race_window) a walk goes
+// through windows of 24 increments, four Philox calls.  A window costs about 440
+// instructions, 430 of them the draws and the bare steps: 24 of them would be
+// needed for each accumulator's tests, so a window runs without tests and is
+// taken again, step by step, only by the walks that may end in it (one window in
+// 120 on the LCA sets).  Time per window and scheduler is 680 cycles, of which
+// the SFU is busy 390.  Measured per launch, ms, 512 sets of 10 000 walks with
+// tests in every step, before and now: LCA (4 accumulators) 22.8 -> 15.3, racing
+// diffusion (3) 12.8 -> 9.8, race with a collapsing bound (4; 190 steps a walk, so
+// half of a warp's windows have a walk that ends) 5.6 -> 5.4.
 #include "common.cuh"
 
 namespace ssm {
@@ -126,13 +135,10 @@ __device__ __forceinline__ float2 std_normal_pair(uint32_t a, uint32_t b) {
     return box_muller(a, b);
 }
 
-// Models with at most 4 accumulators draw a window of WIN steps' normals at
-// once, six per Philox4x32-10 call (bm6_increment), WIN * NP a multiple of six:
-// 2 accumulators 12 steps, 3 accumulators 8, 4 accumulators 6 -- four
-// independent calls per window, whose latencies overlap.  Measured on the
-// 1024-set workloads (ms per launch): LCA 50.3 -> 44.8 and race 19.2 -> 17.0
-// against one call (four normals) per step drawn eight steps ahead, which
-// itself had taken LCA from 66.0 (2 ahead 65.5, 4 ahead 56.3, 8 ahead 52.1).
+// Models with at most 4 accumulators draw a window of WIN steps' increments at
+// once, six per Philox4x32-10 call, WIN * NP a multiple of six: 2 accumulators
+// 12 steps, 3 accumulators 8, 4 accumulators 6 -- four independent calls per
+// window, whose latencies overlap.
 template <int NP> struct RaceWin { static constexpr int value = NP == 2 ? 12 : (NP == 3 ? 8 : 6); };
 
 template <int NP>
@@ -145,45 +151,60 @@ struct RaceLane {
     float x[NP];
 };
 
-// The next window's increments, drawn ahead six per Philox call (calls ctr ..
-// ctr + CALLS - 1) and stored accumulator-major: pre[j * WIN + s] is
-// accumulator j's increment v_j dt + sq_j N(0,1) at step s of the window.
-// WIN is even, so every Box-Muller pair belongs to one accumulator and that
-// accumulator's scale and drift fold into the pair (radius constant
-// c2 = -2 ln(2) sq_j^2, drift v_j dt): a step adds one increment instead of
-// scaling a standard normal and adding the drift.
+// Two accumulators' constants per increment: radius constant c2 = -2 ln(2) sq^2
+// and drift v dt of the steps' increments v dt + sq N(0,1).
+template <int NP> struct RaceScale { float c2[NP], d[NP]; };
+
+// The radius and phase bits of pair i of a call (bm6_increment_pairs' layout).
+__device__ __forceinline__ uint32_t rad_bits(uint4 b, int i) { return i == 0 ? b.x : (i == 1 ? b.y : b.z); }
+__device__ __forceinline__ uint32_t phase_bits(uint4 b, int i) {
+    return i == 0 ? (b.w & 0x007fffffu) : (i == 1 ? phase18(b.w, b.x) : phase18(b.y, b.z));
+}
+
+// The next window's increments, six per Philox call (calls ctr .. ctr + 3),
+// accumulator-major: pre[j * WIN + s] is accumulator j's increment
+// v_j dt + sq_j N(0,1) at step s of the window.  WIN is even, so every
+// Box-Muller pair belongs to one accumulator, whose scale and drift fold into
+// the pair.  Two pairs share the FP32 instructions: those of accumulators j and
+// j + 1 at the same steps, so that a step takes both in one packed operation (an
+// odd last accumulator's pairs go two by two).
 template <int NP>
-__device__ __forceinline__ void draw_window(const RaceParams &p, const RaceLane<NP> &L, const float *vr,
-                                            const float *sr, uint32_t ctr, float *pre) {
-    constexpr int WIN = RaceWin<NP>::value;
-    constexpr int CALLS = WIN * NP / 6;
-    static_assert(WIN % 2 == 0 && (WIN * NP) % 6 == 0, "pairs within one accumulator, whole calls");
-    float c2a[NP], dta[NP];
+__device__ __forceinline__ void draw_window(const RaceParams &p, const RaceLane<NP> &L, const RaceScale<NP> &S,
+                                            uint32_t ctr, float *pre) {
+    constexpr int WIN = RaceWin<NP>::value, H = WIN / 2;
+    static_assert(WIN % 2 == 0 && WIN * NP == 24, "pairs within one accumulator, four calls");
+    uint4 r[4];
 #pragma unroll
-    for (int j = 0; j < NP; ++j) {
-        c2a[j] = -1.3862944f * sr[j] * sr[j];
-        dta[j] = vr[j] * p.dt;
-    }
+    for (int c = 0; c < 4; ++c) r[c] = philox10(make_uint4(ctr + (uint32_t)c, L.n, L.k + p.k_base, 0u), p.key);
 #pragma unroll
-    for (int c = 0; c < CALLS; ++c) {
-        const uint4 r = philox10(make_uint4(ctr + (uint32_t)c, L.n, L.k + p.k_base, 0u), p.key);
-        const float c2[3] = {c2a[(6 * c) / WIN], c2a[(6 * c + 2) / WIN], c2a[(6 * c + 4) / WIN]};
-        const float d[3] = {dta[(6 * c) / WIN], dta[(6 * c + 2) / WIN], dta[(6 * c + 4) / WIN]};
-        bm6_increment_pairs(r, c2, d, pre + 6 * c);
+    for (int q = 0; q < 6; ++q) {
+        // packed operation q works on Box-Muller pairs i0 and i1 of the window's twelve
+        const bool odd = q >= (NP / 2) * H;  // the last of an odd number of accumulators
+        const int j0 = odd ? NP - 1 : 2 * (q / H), j1 = odd ? NP - 1 : j0 + 1;
+        const int i0 = odd ? j0 * H + 2 * (q - (NP / 2) * H) : j0 * H + q % H;
+        const int i1 = odd ? i0 + 1 : j1 * H + q % H;
+        uint64_t cs, sn;
+        bm_pair2(rad_bits(r[i0 / 3], i0 % 3), rad_bits(r[i1 / 3], i1 % 3), phase_bits(r[i0 / 3], i0 % 3),
+                 phase_bits(r[i1 / 3], i1 % 3), pack_f2(S.c2[j0], S.c2[j1]), pack_f2(S.d[j0], S.d[j1]), cs, sn);
+        const float2 c = unpack_f2(cs), t = unpack_f2(sn);
+        pre[2 * i0] = c.x;
+        pre[2 * i0 + 1] = t.x;
+        pre[2 * i1] = c.y;
+        pre[2 * i1 + 1] = t.y;
     }
 }
 
 // True when none of the lane's next `win` steps can reach the step cap or the
 // time limit: the float32 accumulator after (win - 1) more additions of dt is
 // at most t + (win - 1) dt plus their roundings (under dt/4 below 65536 dt),
-// so t + (win + 1) dt <= dl_tmp leaves margin; LCA's float64 accumulator
-// rounds far less.
+// so t + (win + 1) dt <= dl_tmp leaves margin.  LCA's time is exactly steps dt;
+// the margin of 2^-22 covers the two roundings here.
 template <int NP, int FAM>
 __device__ __forceinline__ bool window_clear(const RaceParams &p, const RaceLane<NP> &L, const RaceHead &h,
                                              int win) {
     if (L.ixf + (float)win > h.capf) return false;
     const float span = (float)(win + 1);
-    if (FAM == FAM_LCA) return L.tpd + (double)span * (double)p.dt <= (double)h.dl_tmp;
+    if (FAM == FAM_LCA) return p.dt >= 1e-30f && (L.ixf + span) * (p.dt * 1.00000024f) <= h.dl_tmp;
     return (L.tp < p.dt * 65536.f) && (fmaf(span, p.dt, L.tp) <= h.dl_tmp);
 }
 
@@ -314,6 +335,108 @@ __device__ __forceinline__ bool race_step(const RaceParams &p, RaceLane<NP> &L, 
     return true;
 }
 
+__device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
+
+// Advance a walk by a window of steps whose increments are in pre (draw_window).
+// Returns whether it is still running.  The steps run without a test each: the
+// largest accumulator seen is compared once with the lowest bound of the window
+// (constant and linear bounds; the others compare each step), and only a walk that may
+// have ended, or may reach its time limit, takes the window again step by step.
+template <int NP, int FAM, int BOUND>
+__device__ __forceinline__ bool advance_window(const RaceParams &p, RaceLane<NP> &L, const RaceHead &h,
+                                               const float *pre) {
+    constexpr int WIN = RaceWin<NP>::value;
+    constexpr bool LCA = (FAM == FAM_LCA), ONE_TEST = (BOUND == SSM_BOUND_CONSTANT || BOUND == SSM_BOUND_LINEAR);
+    if (window_clear<NP, FAM>(p, L, h, WIN)) {
+        // accumulators 0 and 1 in x01, 2 and 3 in x23 (2 alone: its upper half is idle)
+        uint64_t xp[(NP + 1) / 2];
+#pragma unroll
+        for (int j = 0; j < NP; j += 2) xp[j / 2] = pack_f2(L.x[j], (j + 1 < NP) ? L.x[j + 1] : 0.f);
+        float tp = L.tp, m = 0.f;
+        bool first = true, below = true;
+        const float c1 = fmaf(h.b - h.g, p.dt, 1.f), c2 = -h.b * p.dt;
+        const uint64_t c1p = pack_f2(c1, c1), c2p = pack_f2(c2, c2);
+#pragma unroll
+        for (int s = 0; s < WIN; ++s) {
+            float x[NP + 1];
+            auto read = [&]() {
+#pragma unroll
+                for (int j = 0; j < NP; j += 2) {
+                    const float2 v = unpack_f2(xp[j / 2]);
+                    x[j] = v.x;
+                    x[j + 1] = v.y;
+                }
+            };
+            auto see = [&]() {
+                if (!ONE_TEST || first) m = fmaxf(x[0], x[1]);
+                else m = max3(m, x[0], x[1]);
+                if (NP == 3) m = fmaxf(m, x[2]);
+                if (NP == 4) m = max3(m, x[2], x[NP - 1]);
+                first = false;
+                if (!ONE_TEST) below &= m <= race_bound<BOUND, false>(h, L.ixf + (float)s, (int)(L.ixf) + s, p, L.k);
+            };
+            read();
+            if (FAM != FAM_RDM) see();
+            if (LCA) {
+                float sum = x[0] + x[1];
+                if (NP >= 3) sum += x[2];
+                if (NP == 4) sum += x[NP - 1];
+                const uint64_t sp = pack_f2(sum, sum);
+#pragma unroll
+                for (int j = 0; j < NP; j += 2) {
+                    if (j + 1 < NP) {
+                        const uint64_t g = pack_f2(pre[j * WIN + s], pre[(j + 1) * WIN + s]);
+                        xp[j / 2] = fma_f2(xp[j / 2], c1p, fma_f2(sp, c2p, g));
+                    } else {
+                        xp[j / 2] = pack_f2(fmaf(x[j], c1, fmaf(sum, c2, pre[j * WIN + s])), 0.f);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < NP; j += 2) {
+                    if (j + 1 < NP) xp[j / 2] = add_f2(xp[j / 2], pack_f2(pre[j * WIN + s], pre[(j + 1) * WIN + s]));
+                    else xp[j / 2] = pack_f2(x[j] + pre[j * WIN + s], 0.f);
+                }
+                tp += p.dt;
+            }
+            if (FAM != FAM_RDM) {
+#pragma unroll
+                for (int j = 0; j < NP; j += 2) {
+                    const float2 v = unpack_f2(xp[j / 2]);
+                    xp[j / 2] = pack_f2(fmaxf(0.f, v.x), (j + 1 < NP) ? fmaxf(0.f, v.y) : 0.f);
+                }
+            } else {
+                read();
+                see();
+            }
+        }
+        if (ONE_TEST) {
+            float lo = race_bound<BOUND, false>(h, L.ixf, 0, p, L.k);
+            if (BOUND == SSM_BOUND_LINEAR)  // rounded monotonically: lowest at one of the ends
+                lo = fminf(lo, race_bound<BOUND, false>(h, L.ixf + (float)(WIN - 1), 0, p, L.k));
+            below = (FAM == FAM_RDM) ? m < lo : m <= lo;
+        }
+        if (below) {
+#pragma unroll
+            for (int j = 0; j < NP; j += 2) {
+                const float2 v = unpack_f2(xp[j / 2]);
+                L.x[j] = v.x;
+                if (j + 1 < NP) L.x[j + 1] = v.y;
+            }
+            L.tp = tp;
+            L.ixf += (float)WIN;
+            return true;
+        }
+    }
+    if (LCA) L.tpd = (double)L.ixf * (double)p.dt;  // exact: 24-bit dt, fewer than 2^29 steps
+    bool live = true;
+    uint32_t unused = 0;
+#pragma unroll
+    for (int s = 0; s < WIN; ++s)
+        if (live) live = race_step<NP, FAM, BOUND, false, false, true, true, WIN>(p, L, h, nullptr, nullptr, NP, unused, pre + s);
+    return live;
+}
+
 template <int NP, int FAM, bool NOISE>
 __device__ __forceinline__ void race_finalize(const RaceParams &p, const RaceLane<NP> &L,
                                               const RaceHead &h, int np) {
@@ -429,6 +552,158 @@ __device__ __forceinline__ bool race_init(const RaceParams &p, RaceLane<NP> &L, 
     return true;
 }
 
+// A trial's RaceScale from its row.
+template <int NP>
+__device__ __forceinline__ void race_scale(const RaceParams &p, const float *row, RaceScale<NP> &S) {
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+        const float sq = __ldg(row + 16 + NP + j);
+        S.c2[j] = -1.3862944f * sq * sq;
+        S.d[j] = __ldg(row + 16 + j) * p.dt;
+    }
+}
+
+// Walks a warp still runs when the queue is empty for its lanes to share their
+// draws (four lanes each at least: a window has four calls).
+constexpr int RACE_SHARE_MAX = 8;
+
+template <int NP, int FAM, int BOUND>
+__global__ void __launch_bounds__(256) k_race_window(const __grid_constant__ RaceParams p) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    const int64_t total = (p.total >= 0) ? p.total : __ldg(p.offsets + p.n_trials) - __ldg(p.offsets);
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    // A launch of at most four walks per warp is spread over all warps, each
+    // taking its walks in one claim: the lanes then share their draws from the start.
+    const int64_t per_warp = (total + warps - 1) / warps;
+    const bool spread = per_warp <= 4;
+    constexpr int np = NP, WIN = RaceWin<NP>::value;
+    __shared__ float drawn[8][32 * 6];  // the last walks' increments, a call of each lane
+    RaceLane<NP> L;
+    RaceHead h;
+    RaceScale<NP> S;
+    L.w = 0; L.k = L.n = 0; L.ixf = L.tp = 0.f; L.tpd = 0.0; L.win = -1;
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+        L.x[j] = 0.f;
+        S.c2[j] = S.d[j] = 0.f;
+    }
+    uint32_t ctr = 0;
+    bool active = false, pending = false, exhausted = false;
+    int64_t q_next = 0, q_end = 0, hint = 0;
+    for (;;) {
+        // ended walks are written and their lanes restarted refill_min at a
+        // time (one divergent pass for several lanes); all at once when the
+        // queue is empty
+        const unsigned need = __ballot_sync(FULL, !active && (!spread || lane < per_warp));
+        const bool pass = exhausted ? (__ballot_sync(FULL, pending) != 0u) : (spread || __popc(need) >= p.refill_min);
+        if (pass && pending) {
+            race_finalize<NP, FAM, false>(p, L, h, np);
+            pending = false;
+        }
+        if (pass && !exhausted) {
+            const int cnt = __popc(need);
+            const int64_t avail = q_end - q_next;
+            int64_t base = 0, claim = 0;
+            if (avail < cnt) {
+                // claims shrink with what is left of the queue, down to the walks
+                // needed now.  Small claims matter here: the longest walks come
+                // first, and a warp with two rounds of them is the launch's end (256
+                // LCA sets: claims of 64 9.6 ms, 32 6.5 ms).
+                claim = max((int64_t)cnt, min((int64_t)p.chunk, (total - q_end) / (2 * warps)));
+                unsigned long long bb = 0ull;
+                if (lane == 0) bb = atomicAdd(&p.hdr->counter, (unsigned long long)claim);
+                base = (int64_t)__shfl_sync(FULL, bb, 0);
+                if (base >= total || spread) exhausted = true;
+            }
+            if (need >> lane & 1u) {
+                const int rank = __popc(need & lt_mask);
+                const int64_t w = (rank < avail) ? q_next + rank : base + (rank - avail);
+                if (w < total && race_init<NP, FAM, false>(p, L, h, w, hint, np)) {
+                    race_scale<NP>(p, p.rows + (int64_t)L.k * p.row_floats, S);
+                    ctr = 0;
+                    active = true;
+                }
+            }
+            if (avail >= cnt) {
+                q_next += cnt;
+            } else {
+                q_next = base + (cnt - avail);
+                q_end = base + claim;
+            }
+        }
+        const unsigned running = __ballot_sync(FULL, active);
+        if (running == 0u || (exhausted && __popc(running) <= RACE_SHARE_MAX)) break;
+        if (active) {
+            float pre[WIN * NP];
+            draw_window<NP>(p, L, S, ctr, pre);
+            ctr += 4;
+            if (!advance_window<NP, FAM, BOUND>(p, L, h, pre)) {
+                active = false;
+                pending = true;
+            }
+        }
+    }
+    // The queue is empty and few of the warp's walks still run: G lanes draw for
+    // each, a Philox call per lane (G / 4 windows), and the walk's own lane takes the
+    // steps.  A walk's lane alone would wait for its four calls one after the other.
+    unsigned running = __ballot_sync(FULL, active);
+    while (running != 0u) {
+        const int m = __popc(running);
+        int G = 4;
+        while (2 * G * m <= 32) G *= 2;
+        const int g = lane / G, call = lane & 3;
+        const int src = (g < m) ? (int)__fns(running, 0u, g + 1) : lane;
+        RaceLane<NP> D;
+        D.n = __shfl_sync(FULL, L.n, src);
+        D.k = __shfl_sync(FULL, L.k, src);
+        uint32_t c = __shfl_sync(FULL, ctr, src) + (uint32_t)(lane & (G - 1));
+        float c2[3] = {0.f, 0.f, 0.f}, d[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            const float cj = __shfl_sync(FULL, S.c2[j], src), dj = __shfl_sync(FULL, S.d[j], src);
+#pragma unroll
+            for (int e = 0; e < 3; ++e)
+                if ((6 * call + 2 * e) / WIN == j) {
+                    c2[e] = cj;
+                    d[e] = dj;
+                }
+        }
+        float *mine = drawn[threadIdx.x >> 5] + lane * 6;
+        const float *walk = drawn[threadIdx.x >> 5] + __popc(running & lt_mask) * G * 6;
+        unsigned now;
+        do {
+            if (g < m) {
+                float x[6];
+                bm6_increment_pairs(philox10(make_uint4(c, D.n, D.k + p.k_base, 0u), p.key), c2, d, x);
+#pragma unroll
+                for (int e = 0; e < 6; ++e) mine[e] = x[e];
+            }
+            c += (uint32_t)G;
+            __syncwarp();
+            if (active) {
+                bool live = true;
+#pragma unroll 1
+                for (int u = 0; u < G / 4 && live; ++u) {
+                    float pre[WIN * NP];
+#pragma unroll
+                    for (int e = 0; e < WIN * NP; ++e) pre[e] = walk[24 * u + e];
+                    live = advance_window<NP, FAM, BOUND>(p, L, h, pre);
+                }
+                ctr += (uint32_t)G;
+                if (!live) {
+                    race_finalize<NP, FAM, false>(p, L, h, np);
+                    active = false;
+                }
+            }
+            __syncwarp();
+            now = __ballot_sync(FULL, active);
+        } while (now == running);
+        running = now;
+    }
+}
+
 template <int NP, int FAM, int BOUND, bool NOISE>
 __global__ void __launch_bounds__(256) k_race(const __grid_constant__ RaceParams p) {
     const unsigned FULL = 0xffffffffu;
@@ -481,10 +756,6 @@ __global__ void __launch_bounds__(256) k_race(const __grid_constant__ RaceParams
             }
         }
         if (__ballot_sync(FULL, active) == 0u) break;
-        // warp-uniform: skip the per-step cap and time tests when no active
-        // lane can reach either within its next window
-        const bool clear = (!NOISE && NP <= 4) &&
-                           __all_sync(FULL, !active || window_clear<NP, FAM>(p, L, h, RaceWin<NP>::value));
         if (active) {
             const float *row = p.rows + (int64_t)L.k * p.row_floats;
             const float *v = row + 16;
@@ -496,32 +767,9 @@ __global__ void __launch_bounds__(256) k_race(const __grid_constant__ RaceParams
                 sr[j] = (j < np) ? __ldg(sq + j) : 0.f;
             }
             bool live = true;
-            if (!NOISE && NP <= 4) {
-                // the next WIN steps' increments first (draw_window), then the
-                // steps; ctr advances per window
-                constexpr int WIN = RaceWin<NP>::value;
-                float nrm[WIN * NP];
-                draw_window<NP>(p, L, vr, sr, ctr, nrm);
-                ctr += WIN * NP / 6;
-                uint32_t unused = 0;
-                if (clear) {
-#pragma unroll
-                    for (int s = 0; s < WIN; ++s)
-                        if (live)
-                            live = race_step<NP, FAM, BOUND, NOISE, false, true, false, WIN>(p, L, h, vr, sr, np,
-                                                                                             unused, nrm + s);
-                } else {
-#pragma unroll
-                    for (int s = 0; s < WIN; ++s)
-                        if (live)
-                            live = race_step<NP, FAM, BOUND, NOISE, false, true, true, WIN>(p, L, h, vr, sr, np,
-                                                                                            unused, nrm + s);
-                }
-            } else {
 #pragma unroll 1
-                for (int s = 0; s < 4 && live; ++s)
-                    live = race_step<NP, FAM, BOUND, NOISE, false>(p, L, h, vr, sr, np, ctr);
-            }
+            for (int s = 0; s < 4 && live; ++s)
+                live = race_step<NP, FAM, BOUND, NOISE, false>(p, L, h, vr, sr, np, ctr);
             if (!live) {
                 active = false;
                 pending = true;
@@ -548,14 +796,16 @@ __global__ void k_race_record(const __grid_constant__ RaceParams p) {
         sr[j] = (j < np) ? row[16 + np + j] : 0.f;
     }
     uint32_t ctr = 0;
-    if (!NOISE && NP <= 4) {
+    if constexpr (!NOISE && NP <= 4) {
         // the main kernel's windows: the same normals in the same order
         constexpr int WIN = RaceWin<NP>::value;
+        RaceScale<NP> S;
+        race_scale<NP>(p, row, S);
         bool live = true;
         while (live) {
             float nrm[WIN * NP];
-            draw_window<NP>(p, L, vr, sr, ctr, nrm);
-            ctr += WIN * NP / 6;
+            draw_window<NP>(p, L, S, ctr, nrm);
+            ctr += 4;
             uint32_t unused = 0;
             for (int s = 0; s < WIN && live; ++s)
                 live = race_step<NP, FAM, BOUND, NOISE, true, true, true, WIN>(p, L, h, vr, sr, np, unused, nrm + s);
@@ -567,8 +817,14 @@ __global__ void k_race_record(const __grid_constant__ RaceParams p) {
 }
 
 template <int NP, int FAM, int BOUND, bool NOISE>
+static auto race_kernel() -> void (*)(const RaceParams) {
+    if constexpr (!NOISE && NP <= 4) return k_race_window<NP, FAM, BOUND>;
+    else return k_race<NP, FAM, BOUND, NOISE>;
+}
+
+template <int NP, int FAM, int BOUND, bool NOISE>
 static int race_launch(const RaceParams &p, const ssm_launch *opt, cudaStream_t st) {
-    auto kern = k_race<NP, FAM, BOUND, NOISE>;
+    auto kern = race_kernel<NP, FAM, BOUND, NOISE>();
     int threads = (opt && opt->block_threads > 0) ? opt->block_threads : 256;
     if (threads > 256 || threads % 32) {
         set_error("block_threads must be a multiple of 32 and at most 256");
@@ -683,7 +939,7 @@ static int run_race(int fam, const float *v, const float *z, const float *t, con
     p.qoff = p.order ? launch->order_offsets : nullptr;
     p.n_trials = n_trials; p.total = total; p.np = np; p.dt = dt; p.smooth = smooth ? 1 : 0;
     p.k_base = (uint32_t)((launch && launch->first_trial > 0) ? launch->first_trial : 0);
-    p.chunk = (launch && launch->chunk >= 32) ? launch->chunk : 64;
+    p.chunk = (launch && launch->chunk >= 32) ? launch->chunk : 32;
     p.refill_min = (launch && launch->refill_min > 0) ? min(launch->refill_min, 32) : SSM_REFILL_MIN_RACE;
     p.table = table; p.tstride = tstride; p.tlen = tlen;
     p.noise = noise; p.nlen = nlen; p.nunif = nunif;
