@@ -508,6 +508,11 @@ int ssm_mlp_forward(const void *image, const float *x, int64_t n, int x_stride,
                     const float *norm_c, const float *norm_s, float *out, float *dx,
                     int dx_stride, int max_ctas, int *status, void *stream);
 
+/* ssm_mlp_forward of the rows (theta[i, 0:5], rt[i], choice[i]) given in three arrays. */
+int ssm_mlp_loglik(const void *image, const float *theta, int theta_stride, const float *rt,
+                   const float *choice, int64_t n, const float *norm_c, const float *norm_s,
+                   float *out, float *dx, int dx_stride, int *status, void *stream);
+
 /*
  * One training gradient: records [n, rec_stride] = (x[0:7], target); loss
  * Huber(delta 1) (loss_kind 0) or squared error (1) times inv_batch, summed.
@@ -524,6 +529,12 @@ int ssm_mlp_train_grad(const void *image, const float *records, int64_t n, int r
 int ssm_mlp_adam(float *params, float *m, float *v, const float *partials, int n_partials,
                  float lr, float beta1, float beta2, float eps, float bias_corr1,
                  float bias_corr2, void *image, void *stream);
+
+/* The same, and *loss = sum of the n_partials loss_partials / n_rows, the batch's mean loss. */
+int ssm_mlp_adam_loss(float *params, float *m, float *v, const float *partials, int n_partials,
+                      float lr, float beta1, float beta2, float eps, float bias_corr1,
+                      float bias_corr2, void *image, const float *loss_partials, int64_t n_rows,
+                      float *loss, void *stream);
 
 #ifdef __cplusplus
 }

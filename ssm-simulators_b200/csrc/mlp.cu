@@ -77,19 +77,32 @@ constexpr int CHUNK = 128 * 16;                 // bytes per 8-column chunk of a
 
 enum Mode { FWD = 0, FWD_DX = 1, TRAIN = 2 };
 template <int MODE> struct Cfg;
+// NWG tiles at a time, SPLIT warpgroups to a tile: both take every row of it, each
+// half of the columns of an epilogue.  The training gradient has shared memory for
+// one tile and, at a batch of 8 192, 64 tiles for 148 SMs: it is bound by the latency
+// of its epilogues' load - compute - store chunks, of which two warpgroups have
+// twice as many in flight (26.1 -> 14.1 us).  The other modes stay with one: forward
+// keeps the SFU busy with a warpgroup for each of its four tiles, and forward + d/dx,
+// split, is no faster (100 000 rows, warm: 31.2 us against 31.2; after an L2 flush the
+// larger code costs 5 us).  Loading the next accumulator chunk while one is worked on
+// gained nothing in any mode (forward, 1 M rows, 107 us against 104).
 template <> struct Cfg<FWD> {
-    static constexpr int NWG = 4;
+    static constexpr int NWG = 4, SPLIT = 1;
     static constexpr int WG_BYTES = TILE_X + TILE_H;                   // X, B0
 };
 template <> struct Cfg<FWD_DX> {
-    static constexpr int NWG = 2;
+    static constexpr int NWG = 2, SPLIT = 1;
     static constexpr int WG_BYTES = TILE_X + TILE_G + TILE_H;          // X, B0, B1
 };
 template <> struct Cfg<TRAIN> {
-    static constexpr int NWG = 1;
+    static constexpr int NWG = 1, SPLIT = 2;
     static constexpr int WG_BYTES = TILE_X + 2 * TILE_H + 2 * TILE_G + TILE_X;  // X H1 H2 H3 G GO
 };
-template <int MODE> constexpr int smem_bytes() { return SM_WG + Cfg<MODE>::NWG * Cfg<MODE>::WG_BYTES; }
+// with two warpgroups to a tile, the first one's partial outputs (a float a row) follow the buffers
+template <int MODE> constexpr int SM_OUT = SM_WG + Cfg<MODE>::NWG * Cfg<MODE>::WG_BYTES;
+template <int MODE> constexpr int smem_bytes() {
+    return SM_OUT<MODE> + (Cfg<MODE>::SPLIT > 1 ? Cfg<MODE>::NWG * 512 : 0);
+}
 static_assert(smem_bytes<FWD>() <= 232448 && smem_bytes<FWD_DX>() <= 232448 &&
               smem_bytes<TRAIN>() <= 232448, "shared memory budget");
 
@@ -255,11 +268,20 @@ __device__ __forceinline__ uint4 ld_row(const uint8_t *tile, int chunk, int r) {
 
 // ------------------------------------------------------------ epilogue pieces
 // x row -> normalised, split hi/lo -> X tile (cols 0-6 hi, 7-13 lo, 14 = 15 = 1).
-__device__ __forceinline__ void stage_x(uint8_t *X, int r, const float *xr, bool valid, const Norm &nm) {
+// An input row: seven floats of x, or (rt given) five of x and one each of rt and choice.
+__device__ __forceinline__ void load_x(const float *x, int x_stride, const float *rt, const float *choice, int64_t row,
+                                       float (&xv)[DIN]) {
+    const float *xr = x + row * (int64_t)x_stride;
+#pragma unroll
+    for (int j = 0; j < DIN - 2; ++j) xv[j] = __ldg(xr + j);
+    xv[DIN - 2] = rt ? __ldg(rt + row) : __ldg(xr + DIN - 2);
+    xv[DIN - 1] = rt ? __ldg(choice + row) : __ldg(xr + DIN - 1);
+}
+__device__ __forceinline__ void stage_x(uint8_t *X, int r, const float (&xv)[DIN], bool valid, const Norm &nm) {
     float hi[7], lo[7];
 #pragma unroll
     for (int j = 0; j < 7; ++j) {
-        const float v = valid ? (xr[j] - nm.c[j]) * nm.s[j] : 0.f;
+        const float v = valid ? (xv[j] - nm.c[j]) * nm.s[j] : 0.f;
         hi[j] = __bfloat162float(__float2bfloat16_rn(v));
         lo[j] = v - hi[j];
     }
@@ -303,20 +325,26 @@ __device__ __forceinline__ void hidden_chunk(int c, uint32_t ta, uint8_t *dst, i
     if (STASH) tmem_st8(ts + 8 * c, p);
 }
 
-template <int NC, int H, int ONES, bool STASH>
-__device__ __forceinline__ void epi_hidden(uint32_t ta, uint8_t *dst, int r, uint32_t ts) {
+// The 16-column chunks [first, last) of n that warpgroup `half` of a tile's SPLIT takes.
+template <int SPLIT> __device__ __forceinline__ int first_chunk(int half, int n) { return SPLIT == 1 ? 0 : half * ((n + 1) / 2); }
+template <int SPLIT> __device__ __forceinline__ int last_chunk(int half, int n) { return SPLIT == 1 || half ? n : (n + 1) / 2; }
+
+template <int NC, int H, int ONES, bool STASH, int SPLIT>
+__device__ __forceinline__ void epi_hidden(uint32_t ta, uint8_t *dst, int r, uint32_t ts, int half) {
     static_assert(H > NC - 16 && ONES >= NC - 16 && ONES + 1 < NC, "padding and ones columns lie in the last chunk");
+    const int end = min(last_chunk<SPLIT>(half, NC / 16), NC / 16 - 1);
 #pragma unroll 1
-    for (int c = 0; c < NC / 16 - 1; ++c) hidden_chunk<false, H, ONES, STASH>(c, ta, dst, r, ts);
-    hidden_chunk<true, H, ONES, STASH>(NC / 16 - 1, ta, dst, r, ts);
+    for (int c = first_chunk<SPLIT>(half, NC / 16); c < end; ++c) hidden_chunk<false, H, ONES, STASH>(c, ta, dst, r, ts);
+    if (SPLIT == 1 || half) hidden_chunk<true, H, ONES, STASH>(NC / 16 - 1, ta, dst, r, ts);
 }
 
 // G = D (TMEM, NC cols) * (1 - h^2) with h read from this row of H; G -> dst
 // (which may alias H); columns [NC, NCPAD) of dst are zeroed.
-template <int NC, int NCPAD>
-__device__ __forceinline__ void epi_dtanh(uint32_t ta, const uint8_t *H, uint8_t *dst, int r) {
+template <int NC, int NCPAD, int SPLIT>
+__device__ __forceinline__ void epi_dtanh(uint32_t ta, const uint8_t *H, uint8_t *dst, int r, int half) {
+    const int end = last_chunk<SPLIT>(half, NC / 16);
 #pragma unroll 1
-    for (int c = 0; c < NC / 16; ++c) {
+    for (int c = first_chunk<SPLIT>(half, NC / 16); c < end; ++c) {
         float v[16];
         tmem_ld16(ta + 16 * c, v);
         const uint4 h0 = ld_row(H, 2 * c, r), h1 = ld_row(H, 2 * c + 1, r);
@@ -331,13 +359,16 @@ __device__ __forceinline__ void epi_dtanh(uint32_t ta, const uint8_t *H, uint8_t
         st_row(dst, 2 * c + 1, r, make_uint4(p[4], p[5], p[6], p[7]));
     }
 #pragma unroll
-    for (int c = NC / 8; c < NCPAD / 8; ++c) st_row(dst, c, r, make_uint4(0, 0, 0, 0));
+    for (int c = NC / 8; c < NCPAD / 8; ++c)
+        if (SPLIT == 1 || half) st_row(dst, c, r, make_uint4(0, 0, 0, 0));
 }
 
 // same, with h taken from the packed bf16 stash in TMEM
-__device__ __forceinline__ void epi_dtanh_stash(uint32_t ta, uint32_t ts, uint8_t *dst, int r) {
+template <int SPLIT>
+__device__ __forceinline__ void epi_dtanh_stash(uint32_t ta, uint32_t ts, uint8_t *dst, int r, int half) {
+    const int end = last_chunk<SPLIT>(half, N1 / 16);
 #pragma unroll 1
-    for (int c = 0; c < N1 / 16; ++c) {
+    for (int c = first_chunk<SPLIT>(half, N1 / 16); c < end; ++c) {
         float v[16];
         tmem_ld16(ta + 16 * c, v);
         uint32_t hh[8];
@@ -356,8 +387,10 @@ __device__ __forceinline__ void epi_dtanh_stash(uint32_t ta, uint32_t ts, uint8_
 // Layer-3 epilogue: h3 = tanh(acc) in fp32 (b3 is in acc), out = b4 + h3 . w4 (fp32),
 // and per KIND: 0 nothing else, 1 G3 = w4 (1 - h3^2) -> dst (d out / d acc3),
 // 2 bf16 h3 with the ones column -> dst (training operand).
-template <int KIND, bool EDGE>
-__device__ __forceinline__ void out_chunk(int c, uint32_t ta, const float4 *w4v, float &o, uint8_t *dst, int r) {
+// With KEEP the tanh values stay in hk and o is left alone.
+template <int KIND, bool EDGE, bool KEEP>
+__device__ __forceinline__ void out_chunk(int c, uint32_t ta, const float4 *w4v, float &o, uint8_t *dst, int r,
+                                          float *hk) {
     float v[16];
     tmem_ld16(ta + 16 * c, v);
     uint32_t p[8];
@@ -373,7 +406,10 @@ __device__ __forceinline__ void out_chunk(int c, uint32_t ta, const float4 *w4v,
             h[3] = tanh_fast(v[4 * q + 3]);
             w[0] = ww.x; w[1] = ww.y; w[2] = ww.z; w[3] = ww.w;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) o = fmaf(w[e], h[e], o);
+            for (int e = 0; e < 4; ++e) {
+                if (KEEP) hk[4 * q + e] = h[e];
+                else o = fmaf(w[e], h[e], o);
+            }
         }
         if (KIND == 1) {
             p[2 * q] = pack2(w[0] * (1.f - h[0] * h[0]), w[1] * (1.f - h[1] * h[1]));
@@ -397,8 +433,34 @@ __device__ __forceinline__ float epi_out(uint32_t ta, const float *w4, float b4,
     const float4 *w4v = reinterpret_cast<const float4 *>(w4);
     float o = b4;
 #pragma unroll 1
-    for (int c = 0; c < N3 / 16 - 1; ++c) out_chunk<KIND, false>(c, ta, w4v, o, dst, r);
-    out_chunk<KIND, true>(N3 / 16 - 1, ta, w4v, o, dst, r);
+    for (int c = 0; c < N3 / 16 - 1; ++c) out_chunk<KIND, false, false>(c, ta, w4v, o, dst, r, nullptr);
+    out_chunk<KIND, true, false>(N3 / 16 - 1, ta, w4v, o, dst, r, nullptr);
+    return o;
+}
+
+// The same by two warpgroups.  The sum goes in the order of the columns, so the
+// first one leaves that of its columns in part[r] and the second one keeps its
+// tanh values in hk, to carry the sum on (out_rest) after the tile's next barrier.
+constexpr int HK = N3 / 2;
+template <int KIND>
+__device__ __forceinline__ void epi_out_half(uint32_t ta, const float *w4, float b4, uint8_t *dst, int r, int half,
+                                             float *part, float (&hk)[HK]) {
+    const float4 *w4v = reinterpret_cast<const float4 *>(w4);
+    float o = b4;
+    if (half == 0) {
+#pragma unroll 1
+        for (int c = 0; c < N3 / 32; ++c) out_chunk<KIND, false, false>(c, ta, w4v, o, dst, r, nullptr);
+        part[r] = o;
+    } else {
+#pragma unroll
+        for (int c = N3 / 32; c < N3 / 16 - 1; ++c)
+            out_chunk<KIND, false, true>(c, ta, w4v, o, dst, r, hk + 16 * (c - N3 / 32));
+        out_chunk<KIND, true, true>(N3 / 16 - 1, ta, w4v, o, dst, r, hk + HK - 16);
+    }
+}
+__device__ __forceinline__ float out_rest(const float *w4, float o, const float (&hk)[HK]) {
+#pragma unroll
+    for (int j = 0; j < H3 - HK; ++j) o = fmaf(w4[HK + j], hk[j], o);
     return o;
 }
 
@@ -408,13 +470,15 @@ __device__ __forceinline__ void flag_error(int *status, int code) {
 
 // ---------------------------------------------------------------- the kernel
 template <int MODE>
-__global__ void __launch_bounds__(128 * Cfg<MODE>::NWG, 1)
-k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n, int x_stride, Norm nm,
+__global__ void __launch_bounds__(128 * Cfg<MODE>::NWG * Cfg<MODE>::SPLIT, 1)
+k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n, int x_stride,
+      const float *__restrict__ rt, const float *__restrict__ choice, Norm nm,
       float *__restrict__ out, float *__restrict__ dx, int dx_stride, int loss_kind, float inv_batch,
       float *__restrict__ part, float *__restrict__ part_loss, int *__restrict__ status) {
-    constexpr int NWG = Cfg<MODE>::NWG;
+    constexpr int NWG = Cfg<MODE>::NWG, SPLIT = Cfg<MODE>::SPLIT, TEAM = 128 * SPLIT;
     extern __shared__ __align__(1024) uint8_t sm[];
-    const int tid = threadIdx.x, wg = tid >> 7, r = tid & 127, warp = tid >> 5;
+    const int tid = threadIdx.x, wg = tid / TEAM, half = (tid >> 7) % SPLIT, r = tid & 127, warp = tid >> 5;
+    const bool lead = tid % TEAM == 0;  // issues the tile's MMAs
     const uint32_t lane = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t s0 = su32(sm);
     const uint32_t wbar = s0 + SM_BAR, mbar = s0 + SM_BAR + 8 * (1 + wg);
@@ -464,16 +528,35 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
     if (!bad) {
         const uint32_t twork = tbase + (MODE == FWD_DX ? 256u * wg : 128u * wg);
         const uint32_t tw = twork + lane;  // this warp's lanes of the work columns
-        for (int64_t tile = (int64_t)blockIdx.x * NWG + wg; tile < n_tiles; tile += (int64_t)gridDim.x * NWG) {
+        float *osum = reinterpret_cast<float *>(sm + SM_OUT<MODE>) + wg * 128;
+        float hk[HK];
+        // Consecutive tiles go to different CTAs, so that a last, partial round has
+        // one tile per SM.  The next tile's inputs are loaded while a tile runs.
+        // (1 M rows, 13.2 rounds: 107 -> 103 us; the SFU's floor is 69.)
+        const int64_t stride = (int64_t)gridDim.x * NWG, first = (int64_t)wg * gridDim.x + blockIdx.x;
+        uint8_t *X = wbuf;
+        const uint32_t Xs = sw;
+        float xv[DIN];
+        if (first < n_tiles) {
+            const int64_t row = first * 128 + r;
+            load_x(x, x_stride, rt, choice, row < n ? row : 0, xv);
+            if (half == 0) stage_x(X, r, xv, row < n, nm);
+        }
+        for (int64_t tile = first; tile < n_tiles; tile += stride) {
             const int64_t row = tile * 128 + r;
             const bool valid = row < n;
-            const float *xr = x + (valid ? row : 0) * (int64_t)x_stride;
-            uint8_t *X = wbuf;
-            const uint32_t Xs = sw;
             int late = 0;
-            stage_x(X, r, xr, valid, nm);
-            fence_async_smem();
-            bar_sync(bid, 128);
+            if (MODE == TRAIN && tile != first && half == 0) {
+                load_x(x, x_stride, rt, choice, valid ? row : 0, xv);
+                stage_x(X, r, xv, valid, nm);
+            }
+            if (MODE == TRAIN || tile == first) {
+                fence_async_smem();
+                bar_sync(bid, TEAM);
+            }
+            const int64_t next = row + stride * 128;
+            const bool more = MODE != TRAIN && half == 0 && tile + stride < n_tiles;
+            if (more) load_x(x, x_stride, rt, choice, next < n ? next : 0, xv);
 
             if (MODE != TRAIN) {
                 // ---------------- inference: forward (and d out / d x)
@@ -485,32 +568,33 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                 const uint32_t Hbs = (MODE == FWD) ? B0s : B1s;
                 const uint32_t tstash = twork + 128u + lane;
 
-                if (r == 0) {
+                if (lead) {
                     tc_after();
                     mma_chain(twork, kmajor(Xs, 128), kmajor(w1s, N1), 1, ID_L12, false);
                     umma_commit(mbar);
                 }
                 late |= !mbar_wait(mbar, phase); phase ^= 1;
                 tc_after();
-                epi_hidden<N1, H1, ONES1, MODE == FWD_DX>(tw, B0, r, tstash);
+                epi_hidden<N1, H1, ONES1, MODE == FWD_DX, SPLIT>(tw, B0, r, tstash, half);
                 if (MODE == FWD_DX) tmem_wait_st();
                 tc_before();
                 fence_async_smem();
-                bar_sync(bid, 128);
+                bar_sync(bid, TEAM);
 
-                if (r == 0) {
+                if (lead) {
                     tc_after();
                     mma_chain(twork, kmajor(B0s, 128), kmajor(w2s, N1), N1 / 16, ID_L12, false);
                     umma_commit(mbar);
                 }
+                if (more) stage_x(X, r, xv, next < n, nm);  // layer 1's MMA has read X
                 late |= !mbar_wait(mbar, phase); phase ^= 1;
                 tc_after();
-                epi_hidden<N2, H2, ONES1, false>(tw, Hb, r, 0);
+                epi_hidden<N2, H2, ONES1, false, SPLIT>(tw, Hb, r, 0, half);
                 tc_before();
                 fence_async_smem();
-                bar_sync(bid, 128);
+                bar_sync(bid, TEAM);
 
-                if (r == 0) {
+                if (lead) {
                     tc_after();
                     mma_chain(twork, kmajor(Hbs, 128), kmajor(w3s, N3), N2 / 16, ID_L3, false);
                     umma_commit(mbar);
@@ -523,33 +607,33 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                 tc_before();
                 if (MODE == FWD_DX) {
                     fence_async_smem();
-                    bar_sync(bid, 128);
+                    bar_sync(bid, TEAM);
                     // D2 = G3 W3 (K = 128 over layer-3 units)
-                    if (r == 0) {
+                    if (lead) {
                         tc_after();
                         mma_chain(twork, kmajor(B0s, 128), mnmajor(w3s, N3), N3 / 16, ID_B112, false);
                         umma_commit(mbar);
                     }
                     late |= !mbar_wait(mbar, phase); phase ^= 1;
                     tc_after();
-                    epi_dtanh<N2, N2>(tw, B1, B1, r);   // G2 over h2, in place
+                    epi_dtanh<N2, N2, SPLIT>(tw, B1, B1, r, half);   // G2 over h2, in place
                     tc_before();
                     fence_async_smem();
-                    bar_sync(bid, 128);
+                    bar_sync(bid, TEAM);
                     // D1 = G2 W2 (K = 112)
-                    if (r == 0) {
+                    if (lead) {
                         tc_after();
                         mma_chain(twork, kmajor(B1s, 128), mnmajor(w2s, N2), N2 / 16, ID_B112, false);
                         umma_commit(mbar);
                     }
                     late |= !mbar_wait(mbar, phase); phase ^= 1;
                     tc_after();
-                    epi_dtanh_stash(tw, tstash, B0, r);  // G1 over h1 (stash) -> B0
+                    epi_dtanh_stash<SPLIT>(tw, tstash, B0, r, half);  // G1 over h1 (stash) -> B0
                     tc_before();
                     fence_async_smem();
-                    bar_sync(bid, 128);
+                    bar_sync(bid, TEAM);
                     // D0 = G1 W1 (K = 112, N = 16)
-                    if (r == 0) {
+                    if (lead) {
                         tc_after();
                         mma_chain(twork, kmajor(B0s, 128), mnmajor(w1s, N1), N1 / 16, ID_B16, false);
                         umma_commit(mbar);
@@ -558,7 +642,7 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                     tc_after();
                     float v[16];
                     tmem_ld16(tw, v);
-                    if (valid) {
+                    if (valid && half == 0) {
                         float *d = dx + row * (int64_t)dx_stride;
 #pragma unroll
                         for (int j = 0; j < DIN; ++j) d[j] = v[j] * nm.s[j];
@@ -573,56 +657,62 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                 const bool acc_dw = any_tile;
                 any_tile = true;
 
-                if (r == 0) {
+                if (lead) {
                     tc_after();
                     mma_chain(twork, kmajor(Xs, 128), kmajor(w1s, N1), 1, ID_L12, false);
                     umma_commit(mbar);
                 }
                 late |= !mbar_wait(mbar, phase); phase ^= 1;
                 tc_after();
-                epi_hidden<N1, H1, ONES1, false>(tw, H1t, r, 0);
+                epi_hidden<N1, H1, ONES1, false, SPLIT>(tw, H1t, r, 0, half);
                 tc_before();
                 fence_async_smem();
-                bar_sync(bid, 128);
+                bar_sync(bid, TEAM);
 
-                if (r == 0) {
+                if (lead) {
                     tc_after();
                     mma_chain(twork, kmajor(H1s, 128), kmajor(w2s, N1), N1 / 16, ID_L12, false);
                     umma_commit(mbar);
                 }
                 late |= !mbar_wait(mbar, phase); phase ^= 1;
                 tc_after();
-                epi_hidden<N2, H2, ONES1, false>(tw, H2t, r, 0);
+                epi_hidden<N2, H2, ONES1, false, SPLIT>(tw, H2t, r, 0, half);
                 tc_before();
                 fence_async_smem();
-                bar_sync(bid, 128);
+                bar_sync(bid, TEAM);
 
-                if (r == 0) {
+                if (lead) {
                     tc_after();
                     mma_chain(twork, kmajor(H2s, 128), kmajor(w3s, N3), N2 / 16, ID_L3, false);
                     umma_commit(mbar);
                 }
                 late |= !mbar_wait(mbar, phase); phase ^= 1;
                 tc_after();
-                const float o = epi_out<2>(tw, w4, bias4, H3t, r);
-                const float y = valid ? xr[DIN] : 0.f;
-                const float e = o - y;
-                float g, l;
-                if (loss_kind == 0) {  // Huber, delta 1
-                    const float ae = fabsf(e);
-                    l = ae <= 1.f ? 0.5f * e * e : ae - 0.5f;
-                    g = fminf(fmaxf(e, -1.f), 1.f);
-                } else {               // squared error
-                    l = e * e;
-                    g = 2.f * e;
+                epi_out_half<2>(tw, w4, bias4, H3t, r, half, osum, hk);
+                bar_sync(bid, TEAM);
+                if (half) {  // the second warpgroup has the output: the row's loss and its gradient
+                    const float o = out_rest(w4, osum[r], hk);
+                    const float y = valid ? x[row * (int64_t)x_stride + DIN] : 0.f;
+                    const float e = o - y;
+                    float g, l;
+                    if (loss_kind == 0) {  // Huber, delta 1
+                        const float ae = fabsf(e);
+                        l = ae <= 1.f ? 0.5f * e * e : ae - 0.5f;
+                        g = fminf(fmaxf(e, -1.f), 1.f);
+                    } else {               // squared error
+                        l = e * e;
+                        g = 2.f * e;
+                    }
+                    if (!valid) { l = 0.f; g = 0.f; }
+                    loss_acc += l;
+                    osum[r] = g * inv_batch;
+                    if (valid && out) out[row] = o;
                 }
-                if (!valid) { l = 0.f; g = 0.f; }
-                loss_acc += l;
-                g *= inv_batch;
-                if (valid && out) out[row] = o;
+                bar_sync(bid, TEAM);
+                const float g = osum[r];
                 // G3 = g w4 (1 - h3^2) -> G ; Gout = (g, 0, ...) -> GO
 #pragma unroll 1
-                for (int c = 0; c < N3 / 8; ++c) {
+                for (int c = half * (N3 / 16); c < (half + 1) * (N3 / 16); ++c) {
                     const uint4 h = ld_row(H3t, c, r);
                     const uint32_t hh[4] = {h.x, h.y, h.z, h.w};
                     uint32_t p[4];
@@ -634,13 +724,12 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                     }
                     st_row(Gt, c, r, make_uint4(p[0], p[1], p[2], p[3]));
                 }
-                st_row(GOt, 0, r, make_uint4(pack2(g, 0.f), 0, 0, 0));
-                st_row(GOt, 1, r, make_uint4(0, 0, 0, 0));
+                st_row(GOt, half, r, make_uint4(half ? 0u : pack2(g, 0.f), 0, 0, 0));
                 tc_before();
                 fence_async_smem();
-                bar_sync(bid, 128);
+                bar_sync(bid, TEAM);
 
-                if (r == 0) {
+                if (lead) {
                     tc_after();
                     // dW4 += H3^T Gout, dW3 += G3^T H2 (K = 128 rows), D2 = G3 W3
                     mma_chain(tbase + T_DW4, mnmajor(H3s, 128), mnmajor(GOs, 128), 8, ID_W16, acc_dw);
@@ -650,12 +739,12 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                 }
                 late |= !mbar_wait(mbar, phase); phase ^= 1;
                 tc_after();
-                epi_dtanh<N2, 128>(tw, H2t, Gt, r);   // G2 -> G (cols 112..127 zero)
+                epi_dtanh<N2, 128, SPLIT>(tw, H2t, Gt, r, half);   // G2 -> G (cols 112..127 zero)
                 tc_before();
                 fence_async_smem();
-                bar_sync(bid, 128);
+                bar_sync(bid, TEAM);
 
-                if (r == 0) {
+                if (lead) {
                     tc_after();
                     mma_chain(tbase + T_DW2, mnmajor(Gs, 128), mnmajor(H1s, 128), 8, ID_W112, acc_dw);
                     mma_chain(twork, kmajor(Gs, 128), mnmajor(w2s, N2), N2 / 16, ID_B112, false);
@@ -663,12 +752,12 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                 }
                 late |= !mbar_wait(mbar, phase); phase ^= 1;
                 tc_after();
-                epi_dtanh<N1, 128>(tw, H1t, Gt, r);   // G1 -> G
+                epi_dtanh<N1, 128, SPLIT>(tw, H1t, Gt, r, half);   // G1 -> G
                 tc_before();
                 fence_async_smem();
-                bar_sync(bid, 128);
+                bar_sync(bid, TEAM);
 
-                if (r == 0) {
+                if (lead) {
                     tc_after();
                     mma_chain(tbase + T_DW1, mnmajor(Gs, 128), mnmajor(Xs, 128), 8, ID_W16, acc_dw);
                     umma_commit(mbar);
@@ -677,7 +766,7 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                 tc_after();
             }
             // every thread of the warpgroup leaves together if any wait expired
-            if (bar_or(bid, 128, late)) {
+            if (bar_or(bid, TEAM, late)) {
                 bad = 1;
                 break;
             }
@@ -686,33 +775,41 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
     if (bad) flag_error(status, SSM_MLP_ERR_TIMEOUT);
 
     if (MODE == TRAIN && !bad) {
-        // per-CTA gradient partials out of TMEM; thread r owns output unit r
+        // per-CTA gradient partials out of TMEM; thread r of both warpgroups owns output
+        // unit r.  Rows of 100 floats start at multiples of four: 16-byte stores
+        // where the caller's buffer allows them.
         float *pp = part + (int64_t)blockIdx.x * PSTRIDE;
         const uint32_t tl = tbase + lane;
-        const bool have = any_tile;
+        const bool have = any_tile, wide = ((uintptr_t)part & 15u) == 0;
+        static_assert(P_W2 % 4 == 0 && P_W3 % 4 == 0 && H1 % 4 == 0 && H2 % 4 == 0 && PSTRIDE % 4 == 0, "rows of float4");
+        auto put = [&](float *rowp, float *biasp, int c, const float (&v)[16]) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int i = 16 * c + 4 * q;
+                const float4 w = have ? make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3])
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (i < H1) {
+                    if (wide) {
+                        *reinterpret_cast<float4 *>(rowp + i) = w;
+                    } else {
+                        rowp[i] = w.x; rowp[i + 1] = w.y; rowp[i + 2] = w.z; rowp[i + 3] = w.w;
+                    }
+                } else if (i == ONES1) {
+                    *biasp = w.x;
+                }
+            }
+        };
+        static_assert(H1 == H2 && H1 == ONES1 && N1 == N2, "dW2 and dW3 rows alike");
+        const int end = last_chunk<SPLIT>(half, N2 / 16);
 #pragma unroll 1
-        for (int c = 0; c < N2 / 16; ++c) {
+        for (int c = first_chunk<SPLIT>(half, N2 / 16); c < end; ++c) {
             float v[16];
             tmem_ld16(tl + T_DW2 + 16 * c, v);
-            if (r < H2) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int i = 16 * c + j;
-                    if (i < H1) pp[P_W2 + r * H1 + i] = have ? v[j] : 0.f;
-                    else if (i == ONES1) pp[P_B2 + r] = have ? v[j] : 0.f;
-                }
-            }
+            if (r < H2) put(pp + P_W2 + r * H1, pp + P_B2 + r, c, v);
             tmem_ld16(tl + T_DW3 + 16 * c, v);
-            if (r < H3) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int i = 16 * c + j;
-                    if (i < H2) pp[P_W3 + r * H2 + i] = have ? v[j] : 0.f;
-                    else if (i == ONES1) pp[P_B3 + r] = have ? v[j] : 0.f;
-                }
-            }
+            if (r < H3) put(pp + P_W3 + r * H2, pp + P_B3 + r, c, v);
         }
-        {
+        if (half) {
             float v[16];
             tmem_ld16(tl + T_DW1, v);
             if (r < H1) {
@@ -724,13 +821,13 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
             if (r < H3) pp[P_W4 + r] = have ? v[0] : 0.f;
             if (r == ONES3) pp[P_B4] = have ? v[0] : 0.f;
         }
-        // CTA loss sum (one warpgroup): warp shuffle, then four warp sums
+        // CTA loss sum (the second warpgroup's): warp shuffle, then four warp sums
         float s = loss_acc;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         float *red = reinterpret_cast<float *>(sm + SM_BAR + 96);
-        if ((tid & 31) == 0) red[warp] = s;
-        bar_sync(1, 128);
+        if (half && (tid & 31) == 0) red[warp & 3] = s;
+        bar_sync(1, TEAM);
         if (tid == 0) part_loss[blockIdx.x] = red[0] + red[1] + red[2] + red[3];
     }
 
@@ -791,13 +888,28 @@ __global__ void k_mlp_pack(const float *__restrict__ p, uint8_t *__restrict__ im
 }
 
 // Adam over the summed per-CTA partials (fixed CTA order: deterministic), then
-// refresh the parameter's places in the bf16 image.
+// refresh the parameter's places in the bf16 image.  With `loss` one block more
+// sums the CTAs' losses into *loss = sum / n_rows, which two launches did before
+// (a step on 8 192 records: 42 -> 28 us, the split training gradient included;
+// what is left is the host's work for the two launches).
 __global__ void k_mlp_adam(float *__restrict__ p, float *__restrict__ m, float *__restrict__ v,
                            const float *__restrict__ part, int n_part, float lr, float b1, float b2, float eps,
-                           float bc1, float bc2, uint8_t *__restrict__ image) {
+                           float bc1, float bc2, uint8_t *__restrict__ image, const float *__restrict__ part_loss,
+                           float n_rows, float *__restrict__ loss) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (loss && blockIdx.x == gridDim.x - 1) {
+        if (threadIdx.x < 32) {
+            float t = 0.f;
+            for (int c = threadIdx.x; c < n_part; c += 32) t += part_loss[c];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (threadIdx.x == 0) *loss = t / n_rows;
+        }
+        return;
+    }
     if (i >= NPARAMS) return;
     float g = 0.f;
+#pragma unroll 16
     for (int c = 0; c < n_part; ++c) g += part[(int64_t)c * PSTRIDE + i];
     const float mi = b1 * m[i] + (1.f - b1) * g;
     const float vi = b2 * v[i] + (1.f - b2) * g * g;
@@ -837,7 +949,8 @@ __global__ void k_mlp_adam(float *__restrict__ p, float *__restrict__ m, float *
 }
 
 template <int MODE>
-static int launch(const void *image, const float *x, int64_t n, int x_stride, const float *nc, const float *ns,
+static int launch(const void *image, const float *x, int64_t n, int x_stride, const float *rt, const float *choice,
+                  const float *nc, const float *ns,
                   float *out, float *dx, int dx_stride, int loss_kind, float inv_batch, float *part,
                   float *part_loss, int grid, int *status, cudaStream_t st) {
     static bool configured[64] = {false};
@@ -852,8 +965,8 @@ static int launch(const void *image, const float *x, int64_t n, int x_stride, co
         nm.c[j] = (j < DIN && nc) ? nc[j] : 0.f;
         nm.s[j] = (j < DIN && ns) ? ns[j] : 1.f;
     }
-    k_mlp<MODE><<<grid, 128 * Cfg<MODE>::NWG, smem_bytes<MODE>(), st>>>(
-        (const uint8_t *)image, x, n, x_stride, nm, out, dx, dx_stride, loss_kind, inv_batch, part, part_loss,
+    k_mlp<MODE><<<grid, 128 * Cfg<MODE>::NWG * Cfg<MODE>::SPLIT, smem_bytes<MODE>(), st>>>(
+        (const uint8_t *)image, x, n, x_stride, rt, choice, nm, out, dx, dx_stride, loss_kind, inv_batch, part, part_loss,
         status);
     SSM_CUDA(cudaGetLastError());
     return SSM_OK;
@@ -875,6 +988,20 @@ int ssm_mlp_pack(const float *params, void *image, void *stream) {
     return SSM_OK;
 }
 
+static int mlp_forward(const void *image, const float *x, int64_t n, int x_stride, const float *rt,
+                       const float *choice, const float *norm_c, const float *norm_s, float *out, float *dx,
+                       int dx_stride, int max_ctas, int *status, void *stream) {
+    const int64_t tiles = (n + 127) / 128;
+    int grid = (int)std::min<int64_t>(tiles, (int64_t)sm_count());
+    if (max_ctas > 0) grid = std::min(grid, max_ctas);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (dx)
+        return launch<FWD_DX>(image, x, n, x_stride, rt, choice, norm_c, norm_s, out, dx, dx_stride, 0, 0.f, nullptr,
+                              nullptr, grid, status, st);
+    return launch<FWD>(image, x, n, x_stride, rt, choice, norm_c, norm_s, out, nullptr, 0, 0, 0.f, nullptr, nullptr,
+                       grid, status, st);
+}
+
 int ssm_mlp_forward(const void *image, const float *x, int64_t n, int x_stride, const float *norm_c,
                     const float *norm_s, float *out, float *dx, int dx_stride, int max_ctas, int *status,
                     void *stream) {
@@ -884,16 +1011,21 @@ int ssm_mlp_forward(const void *image, const float *x, int64_t n, int x_stride, 
     SSM_REQUIRE(((uintptr_t)image & 15) == 0, "ssm_mlp_forward: image must be 16-byte aligned");
     SSM_REQUIRE(x_stride >= DIN, "ssm_mlp_forward: x_stride < 7");
     SSM_REQUIRE(!dx || dx_stride >= DIN, "ssm_mlp_forward: dx_stride < 7");
-    const int64_t tiles = (n + 127) / 128;
-    const int nwg = dx ? Cfg<FWD_DX>::NWG : Cfg<FWD>::NWG;
-    int grid = (int)std::min<int64_t>((tiles + nwg - 1) / nwg, (int64_t)sm_count());
-    if (max_ctas > 0) grid = std::min(grid, max_ctas);
-    cudaStream_t st = (cudaStream_t)stream;
-    if (dx)
-        return launch<FWD_DX>(image, x, n, x_stride, norm_c, norm_s, out, dx, dx_stride, 0, 0.f, nullptr, nullptr,
-                              grid, status, st);
-    return launch<FWD>(image, x, n, x_stride, norm_c, norm_s, out, nullptr, 0, 0, 0.f, nullptr, nullptr, grid,
-                       status, st);
+    return mlp_forward(image, x, n, x_stride, nullptr, nullptr, norm_c, norm_s, out, dx, dx_stride, max_ctas, status,
+                       stream);
+}
+
+int ssm_mlp_loglik(const void *image, const float *theta, int theta_stride, const float *rt, const float *choice,
+                   int64_t n, const float *norm_c, const float *norm_s, float *out, float *dx, int dx_stride,
+                   int *status, void *stream) {
+    SSM_REQUIRE(n >= 0, "ssm_mlp_loglik: n < 0");
+    if (n == 0) return SSM_OK;
+    SSM_REQUIRE(image && theta && rt && choice && out, "ssm_mlp_loglik: null pointer");
+    SSM_REQUIRE(((uintptr_t)image & 15) == 0, "ssm_mlp_loglik: image must be 16-byte aligned");
+    SSM_REQUIRE(theta_stride >= DIN - 2, "ssm_mlp_loglik: theta_stride < 5");
+    SSM_REQUIRE(!dx || dx_stride >= DIN, "ssm_mlp_loglik: dx_stride < 7");
+    return mlp_forward(image, theta, n, theta_stride, rt, choice, norm_c, norm_s, out, dx, dx_stride, 0, status,
+                       stream);
 }
 
 int ssm_mlp_train_grad(const void *image, const float *records, int64_t n, int rec_stride, const float *norm_c,
@@ -905,18 +1037,34 @@ int ssm_mlp_train_grad(const void *image, const float *records, int64_t n, int r
     SSM_REQUIRE(rec_stride >= DIN + 1, "ssm_mlp_train_grad: rec_stride < 8");
     SSM_REQUIRE(loss_kind == 0 || loss_kind == 1, "ssm_mlp_train_grad: loss_kind must be 0 (huber) or 1 (mse)");
     SSM_REQUIRE(n_ctas > 0, "ssm_mlp_train_grad: n_ctas must be positive");
-    return launch<TRAIN>(image, records, n, rec_stride, norm_c, norm_s, out, nullptr, 0, loss_kind, inv_batch,
+    return launch<TRAIN>(image, records, n, rec_stride, nullptr, nullptr, norm_c, norm_s, out, nullptr, 0, loss_kind, inv_batch,
                          partials, loss_partials, n_ctas, status, (cudaStream_t)stream);
+}
+
+static int mlp_adam(float *params, float *m, float *v, const float *partials, int n_partials, float lr, float beta1,
+                    float beta2, float eps, float bias_corr1, float bias_corr2, void *image,
+                    const float *loss_partials, float n_rows, float *loss, void *stream) {
+    SSM_REQUIRE(params && m && v && partials && image, "ssm_mlp_adam: null pointer");
+    SSM_REQUIRE(n_partials > 0, "ssm_mlp_adam: n_partials must be positive");
+    k_mlp_adam<<<(NPARAMS + 255) / 256 + (loss ? 1 : 0), 256, 0, (cudaStream_t)stream>>>(
+        params, m, v, partials, n_partials, lr, beta1, beta2, eps, bias_corr1, bias_corr2, (uint8_t *)image,
+        loss_partials, n_rows, loss);
+    SSM_CUDA(cudaGetLastError());
+    return SSM_OK;
 }
 
 int ssm_mlp_adam(float *params, float *m, float *v, const float *partials, int n_partials, float lr, float beta1,
                  float beta2, float eps, float bias_corr1, float bias_corr2, void *image, void *stream) {
-    SSM_REQUIRE(params && m && v && partials && image, "ssm_mlp_adam: null pointer");
-    SSM_REQUIRE(n_partials > 0, "ssm_mlp_adam: n_partials must be positive");
-    k_mlp_adam<<<(NPARAMS + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-        params, m, v, partials, n_partials, lr, beta1, beta2, eps, bias_corr1, bias_corr2, (uint8_t *)image);
-    SSM_CUDA(cudaGetLastError());
-    return SSM_OK;
+    return mlp_adam(params, m, v, partials, n_partials, lr, beta1, beta2, eps, bias_corr1, bias_corr2, image,
+                    nullptr, 1.f, nullptr, stream);
+}
+
+int ssm_mlp_adam_loss(float *params, float *m, float *v, const float *partials, int n_partials, float lr,
+                      float beta1, float beta2, float eps, float bias_corr1, float bias_corr2, void *image,
+                      const float *loss_partials, int64_t n_rows, float *loss, void *stream) {
+    SSM_REQUIRE(loss_partials && loss && n_rows > 0, "ssm_mlp_adam_loss: null pointer or no rows");
+    return mlp_adam(params, m, v, partials, n_partials, lr, beta1, beta2, eps, bias_corr1, bias_corr2, image,
+                    loss_partials, (float)n_rows, loss, stream);
 }
 
 }  // extern "C"

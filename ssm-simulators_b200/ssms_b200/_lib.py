@@ -112,6 +112,8 @@ _SIGNATURES: dict[str, tuple] = {
     "ssm_mlp_forward": (_I, [_P, _P, _I64, _I, _P, _P, _P, _P, _I, _I, _P, _P]),
     "ssm_mlp_train_grad": (_I, [_P, _P, _I64, _I, _P, _P, _I, _F, _P, _P, _P, _I, _P, _P]),
     "ssm_mlp_adam": (_I, [_P, _P, _P, _P, _I, _F, _F, _F, _F, _F, _F, _P, _P]),
+    "ssm_mlp_adam_loss": (_I, [_P, _P, _P, _P, _I, _F, _F, _F, _F, _F, _F, _P, _P, _I64, _P, _P]),
+    "ssm_mlp_loglik": (_I, [_P, _P, _I, _P, _P, _I64, _P, _P, _P, _P, _I, _P, _P]),
 }
 
 MLP_NPARAMS = 23141

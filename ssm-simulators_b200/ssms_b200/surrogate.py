@@ -173,10 +173,14 @@ class MlpSurrogate:
 
     def loglik(self, theta, rt, choice) -> torch.Tensor:
         """Differentiable log-likelihood (theta [n, 5], rt [n], choice [n])."""
-        theta = torch.as_tensor(theta, dtype=torch.float32, device=self.params.device)
-        rt = torch.as_tensor(rt, dtype=torch.float32, device=self.params.device).reshape(-1, 1)
-        choice = torch.as_tensor(choice, dtype=torch.float32, device=self.params.device).reshape(-1, 1)
-        return SurrogateLogLik.apply(torch.cat([theta.reshape(-1, DIN - 2), rt, choice], dim=1), self)
+        dev = self.params.device
+        theta = torch.as_tensor(theta, dtype=torch.float32, device=dev).reshape(-1, DIN - 2)
+        rt = torch.as_tensor(rt, dtype=torch.float32, device=dev).reshape(-1)
+        choice = torch.as_tensor(choice, dtype=torch.float32, device=dev).reshape(-1)
+        if not theta.shape[0] == rt.shape[0] == choice.shape[0]:
+            raise RuntimeError(f"theta, rt and choice must have as many rows: {theta.shape[0]}, {rt.shape[0]}, "
+                               f"{choice.shape[0]}")
+        return _LogLikColumns.apply(theta, rt, choice, self)
 
     # ------------------------------------------------------------- training
     def _buffers(self, n_ctas: int):
@@ -210,11 +214,12 @@ class MlpSurrogate:
         part, lpart, n_ctas = self.grad(records)
         self.step += 1
         b1, b2 = betas
-        _lib.check(_lib.lib().ssm_mlp_adam(
+        loss = torch.empty((), dtype=torch.float32, device=self.params.device)
+        _lib.check(_lib.lib().ssm_mlp_adam_loss(
             D.ptr(self.params), D.ptr(self.m), D.ptr(self.v), D.ptr(part), n_ctas, float(lr), float(b1),
             float(b2), float(eps), float(1.0 - b1 ** self.step), float(1.0 - b2 ** self.step),
-            D.ptr(self.image), D.stream_ptr()))
-        return lpart[:n_ctas].sum() / records.shape[0]
+            D.ptr(self.image), D.ptr(lpart), records.shape[0], D.ptr(loss), D.stream_ptr()))
+        return loss
 
     def prepare_records(self, data_or_records) -> torch.Tensor:
         """Training records on the device, labels raised to the lower bound.
@@ -283,6 +288,34 @@ class SurrogateLogLik(torch.autograd.Function):
     def backward(ctx, gout):
         (dx,) = ctx.saved_tensors
         return gout.reshape(-1, 1) * dx, None
+
+
+class _LogLikColumns(torch.autograd.Function):
+    """The same from theta [n, 5], rt [n] and choice [n] in their own arrays: the
+    kernel reads them there, without a joined copy (and its backward) of the rows."""
+
+    @staticmethod
+    def forward(ctx, theta, rt, choice, net: MlpSurrogate):
+        th, r, c = theta.detach().contiguous(), rt.detach().contiguous(), choice.detach().contiguous()
+        n = th.shape[0]
+        out = torch.empty(n, dtype=torch.float32, device=th.device)
+        want = any(ctx.needs_input_grad[:3])
+        dx = torch.empty(n, DIN, dtype=torch.float32, device=th.device) if want else None
+        if n:
+            _lib.check(_lib.lib().ssm_mlp_loglik(
+                D.ptr(net.image), D.ptr(th), DIN - 2, D.ptr(r), D.ptr(c), n, net._nc, net._ns, D.ptr(out),
+                D.ptr(dx), DIN, D.ptr(net.status), D.stream_ptr()))
+        if want:
+            ctx.save_for_backward(dx)
+        return out
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, gout):
+        (dx,) = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        return (gout.reshape(-1, 1) * dx[:, :DIN - 2] if need[0] else None,
+                gout * dx[:, DIN - 2] if need[1] else None, gout * dx[:, DIN - 1] if need[2] else None, None)
 
 
 class LikelihoodEstimator:
