@@ -113,12 +113,18 @@ int ssm_simulator_summary(const float *rts, const int32_t *choices, int64_t n_sa
     SSM_REQUIRE(choice_values && edges_a && edges_b && choice_counts && kept_counts && omission_counts &&
                 nogo_counts && hist_a && hist_b, "all buffers are required");
     cudaStream_t st = (cudaStream_t)stream;
-    SSM_CUDA(cudaMemsetAsync(choice_counts, 0, sizeof(int64_t) * n_trials * n_choices, st));
-    SSM_CUDA(cudaMemsetAsync(kept_counts, 0, sizeof(int64_t) * n_trials * n_choices, st));
-    SSM_CUDA(cudaMemsetAsync(omission_counts, 0, sizeof(int64_t) * n_trials, st));
-    SSM_CUDA(cudaMemsetAsync(nogo_counts, 0, sizeof(int64_t) * n_trials, st));
-    SSM_CUDA(cudaMemsetAsync(hist_a, 0, sizeof(int64_t) * nbins_a * n_choices, st));
-    SSM_CUDA(cudaMemsetAsync(hist_b, 0, sizeof(int64_t) * nbins_b * n_choices, st));
+    // Outputs that lie one after the other are cleared at once (500 trials of one
+    // sample: six clears took 10 us of a kernel of 8).
+    int64_t *const outs[6] = {choice_counts, kept_counts, omission_counts, nogo_counts, hist_a, hist_b};
+    const int64_t sizes[6] = {n_trials * n_choices, n_trials * n_choices, n_trials, n_trials,
+                              (int64_t)nbins_a * n_choices, (int64_t)nbins_b * n_choices};
+    for (int i = 0; i < 6;) {
+        int64_t count = sizes[i];
+        int k = i + 1;
+        while (k < 6 && outs[k] == outs[i] + count) count += sizes[k++];
+        SSM_CUDA(cudaMemsetAsync(outs[i], 0, sizeof(int64_t) * count, st));
+        i = k;
+    }
     if (n_samples == 0 || n_trials == 0) return SSM_OK;
     SSM_REQUIRE(rts && choices, "rts and choices are required");
     SSM_REQUIRE(n_trials < (1ll << 31), "too many trials for one launch");

@@ -393,18 +393,24 @@ def summarize_output(rts, choices, n_samples: int, n_trials: int, possible_choic
     from . import _lib
 
     dev = Dv.require_cuda()
-    C = len(possible_choices)
-    r = torch.from_numpy(np.ascontiguousarray(np.asarray(rts, np.float32).reshape(-1))).to(dev)
-    c = torch.from_numpy(np.ascontiguousarray(np.asarray(choices).astype(np.int32).reshape(-1))).to(dev)
-    cv = torch.from_numpy(np.asarray(possible_choices, np.int32)).to(dev)
-    ea = torch.from_numpy(_hist_edges(128, float(max_t))).to(dev)
-    eb = torch.from_numpy(_hist_edges(256, float(max_t))).to(dev)
-    i64 = lambda *shape: torch.empty(*shape, dtype=torch.int64, device=dev)  # noqa: E731
-    cc, kc, om, ng, ha, hb = i64(n_trials * C), i64(n_trials * C), i64(n_trials), i64(n_trials), i64(128 * C), i64(256 * C)
+    C, K, n = len(possible_choices), int(n_trials), int(np.size(rts))
+    # inputs and counts are one array each: a copy synchronises, so one in and one out
+    at_cv = 8 * (129 + 257)
+    at_r = at_cv + (4 * C + 15) // 16 * 16
+    at_c = at_r + (4 * n + 15) // 16 * 16
+    host = np.empty(at_c + 4 * n, np.uint8)
+    host[:8 * 129].view(np.float64)[:] = _hist_edges(128, float(max_t))
+    host[8 * 129:at_cv].view(np.float64)[:] = _hist_edges(256, float(max_t))
+    host[at_cv:at_cv + 4 * C].view(np.int32)[:] = possible_choices
+    host[at_r:at_r + 4 * n].view(np.float32)[:] = np.asarray(rts).reshape(-1)
+    host[at_c:].view(np.int32)[:] = np.asarray(choices).reshape(-1)
+    src = torch.from_numpy(host).to(dev)
+    counts = torch.empty(K * (2 * C + 2) + 384 * C, dtype=torch.int64, device=dev)
+    p, q = Dv.ptr(src), Dv.ptr(counts)
+    at = np.cumsum([0, K * C, K * C, K, K, 128 * C, 256 * C])
     _lib.check(_lib.lib().ssm_simulator_summary(
-        Dv.ptr(r), Dv.ptr(c), int(n_samples), int(n_trials), Dv.ptr(cv), C, Dv.ptr(ea), 128, Dv.ptr(eb), 256,
-        Dv.ptr(cc), Dv.ptr(kc), Dv.ptr(om), Dv.ptr(ng), Dv.ptr(ha), Dv.ptr(hb), Dv.stream_ptr()))
-    h = lambda t, *shape: t.cpu().numpy().reshape(*shape)  # noqa: E731
-    return {"choice": h(cc, n_trials, C).astype(np.float64), "kept": h(kc, n_trials, C).astype(np.float64),
-            "omission": h(om, n_trials).astype(np.float64), "nogo": h(ng, n_trials).astype(np.float64),
-            "binned_128": h(ha, 128, C).astype(np.float64), "binned_256": h(hb, 256, C).astype(np.float64)}
+        p + at_r, p + at_c, int(n_samples), K, p + at_cv, C, p, 128, p + 8 * 129, 256,
+        *(q + 8 * int(o) for o in at[:6]), Dv.stream_ptr()))
+    cc, kc, om, ng, ha, hb = np.split(counts.cpu().numpy().astype(np.float64), at[1:6])
+    return {"choice": cc.reshape(K, C), "kept": kc.reshape(K, C), "omission": om, "nogo": ng,
+            "binned_128": ha.reshape(128, C), "binned_256": hb.reshape(256, C)}
