@@ -84,7 +84,7 @@ def expected_walk_time(v, a, z, s=1.0, *, legacy: bool = False, bound_kind: int 
             y0 = (2 * z - 1) * a
             shrink = 0.7 * np.minimum(slope, 0.0)
             lo, hi = np.zeros(K), np.minimum(e, cap)
-            for _ in range(40):
+            for _ in range(24):  # to hi / 2^24: far below a step
                 mid = 0.5 * (lo + hi)
                 a_eff = np.maximum(a + shrink * mid, 1e-3)
                 x_eff = np.clip(y0 + a_eff, 1e-9, 2 * a_eff - 1e-9)

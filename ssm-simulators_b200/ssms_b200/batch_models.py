@@ -146,16 +146,18 @@ class SetBatch:
         else:
             raise ValueError(f"no batched device path for simulator {sim_name!r}")
         self.lanes_per_walk = 0
+        est = None
         if sim_name in SINGLE and wide_family(sim_name, self.kind):
             cap = np.minimum(float(max_t), np.maximum(np.asarray(_col(kwargs["deadline"], K), np.float64)
                                                       - np.asarray(_col(kwargs["t"], K), np.float64), 0.0))
-            e, walk_cap = expected_walk_time(
+            est, walk_cap = expected_walk_time(
                 _col(kwargs["v"], K), spec["a"], _col(kwargs["z"], K), _col(kwargs["s"], K),
                 legacy=sim_name == "ddm", bound_kind=self.kind, p1=spec["p1"], p2=spec["p2"], t_cap=cap,
                 return_cap=True)
-            self.lanes_per_walk = lanes_per_walk_for(e, walk_cap, ns, delta_t)
-        est = expected_set_time(sim_name, kwargs, spec, K, max_t) if K > 1 else None
-        if est is not None:  # sets longest-first (outputs do not depend on the order)
+            self.lanes_per_walk = lanes_per_walk_for(est, walk_cap, ns, delta_t)
+        elif K > 1:
+            est = expected_set_time(sim_name, kwargs, spec, K, max_t)
+        if est is not None and K > 1:  # sets longest-first (outputs do not depend on the order)
             o, q = longest_first(est, ns)
             self.order_t, self.qoff_t = torch.from_numpy(o).cuda(), torch.from_numpy(q).cuda()
 
