@@ -47,50 +47,48 @@ WORKLOAD = ("ddm_flexbound angle boundary, 4096 theta ~ U(v[-3,3], a[0.3,3], z[0
 # accumulator-step of the algorithm as implemented, with no block, queue or
 # per-walk overhead.  Philox4x32-10: 10 rounds x (2 wide multiplies + 2
 # three-input XORs) + the counter = 42 instructions per call, six increments
-# per call -> 7; Box-Muller: 14 per pair (radius: bits to float, shift,
-# log2, scale, sqrt = 5; phase: bit assembly 3 on average, range scale, the
-# SFU's argument scaling, sin, cos = 7; two fused multiply-adds) -> 7; the
-# step with the per-block time test passing: moving bound, compare folded
-# with the walk's predicate, position and time updates -> 4.  Total 18.
-# (The four-per-call layout this kernel replaced needed 22: 10.5 + 6 + 5.5.)
-INSTR_PER_STEP = 18.0
+# per call -> 7; Box-Muller: 10.8 per pair (log2, sqrt, sin, cos, the SFU's
+# argument scaling, bits to float, 2.3 of phase bit assembly on average = 8.3;
+# shift, scale, range scale and the two fused multiply-adds packed, an
+# instruction for two pairs = 2.5) -> 5.4; the step with the per-block time
+# test passing: moving bound, compare folded with the walk's predicate,
+# position and time updates -> 4.  Total 16.4 (18 without packed FP32).
+INSTR_PER_STEP = 16.4
 
 # The same accounting for the other benchmarked families, per accumulator-step
 # (lane-instructions, no block, queue or per-walk overhead).  The
 # single-accumulator Gaussian models draw six increments per Philox call
-# (7 + 7 = 14 per increment, folded scale and drift) and test the time once per
-# block (constant-bound step 3: compare with predicate, position and time
-# updates); the race family draws six per call too (14 per normal, each
-# accumulator's scale and drift folded into its pairs) and tests the time
-# every step; ddm_flex draws six per call as well and tests the time every step
+# (7 + 5.4 = 12.4 per increment, folded scale and drift) and test the time once
+# per block (constant-bound step 3: compare with predicate, position and time
+# updates); the race family draws six per call too (12.4 per normal, each
+# accumulator's scale and drift folded into its pairs) and tests bound and time
+# once per window of 24 increments; ddm_flex draws six per call as well
 # (constant-bound step 4.5, 5.5 against a moving bound).
 INSTR_MIN = {
-    # constant bound: 16.5 + 4.5
-    "plain_ddm": (17.0, "Gaussian increment 14 (six per Philox call) + constant-bound step 3"),
-    "full_ddm": (17.0, "Gaussian increment 14 + constant-bound step 3 (per-walk draws amortised)"),
+    "plain_ddm": (15.4, "Gaussian increment 12.4 (six per Philox call) + constant-bound step 3"),
+    "full_ddm": (15.4, "Gaussian increment 12.4 + constant-bound step 3 (per-walk draws amortised)"),
     # the leaky update y (1 - g dt) + increment is one FFMA, like the plain add
-    "ornstein": (17.0, "Gaussian increment 14 + constant-bound step 3 (leak folded into one FFMA)"),
+    "ornstein": (15.4, "Gaussian increment 12.4 + constant-bound step 3 (leak folded into one FFMA)"),
     # drift table: one FFMA v(t) dt + increment, a 16-byte load per four steps
-    "conflict_ds": (19.75, "Gaussian increment 14 (six per Philox call) + constant-bound step 4.5 "
+    "conflict_ds": (18.15, "Gaussian increment 12.4 (six per Philox call) + constant-bound step 4.5 "
                            "+ drift-table FFMA 1 + vector load 0.25"),
     # two Philox words per stable variate (21), Chambers-Mallows-Stuck with
-    # reduced-angle polynomials: uniform and fold 5, W = -ln u 5, three
-    # polynomial sin/cos 23, three log2 + exponent + ex2 7, product, sign,
-    # clamp and NaN guard 6, scale FFMA 1 = 47; constant-bound step 3 (time
-    # tested once per block)
-    "levy": (71.0, "Philox 21 (two words per variate) + CMS 47 + constant-bound step 3"),
-    # per accumulator: increment 14 (scale and drift folded in), add + clamp at
-    # 0 + threshold compare 3; per step over 4 accumulators: moving bound, time
-    # update and test, predicate 3.5 / 4
-    "race_no_bias_angle_4": (17.875, "normal 14 (six per Philox call) + add, clamp, compare 3 "
-                                     "+ shared step 3.5/4"),
-    # per accumulator: increment 14 (v dt + s sqrt(dt) N), the update
-    # x (1 - g dt + b dt) + S (-b dt) + increment as two FFMA, clamp 1,
-    # compare 1; the sum S 3/4; per step the float64 time update, test and
-    # predicate 3 / 4
-    "lca_no_bias_4": (19.5, "increment 14 + LCA update 2 + clamp, compare 2 + sum 0.75 + shared step 3/4"),
-    # per accumulator: increment 14, add + compare 2; shared step 3.5 / 3
-    "racing_diffusion_3": (17.17, "increment 14 + add, compare 2 + shared step 3.5/3"),
+    # reduced-angle polynomials, two variates to a packed FP32 instruction:
+    # uniform and fold 3.5, W = -ln u 4, three polynomial sin/cos 11.5, three
+    # log2 + exponent + ex2 6, product, sign, clamp and NaN guard 5, scale FFMA
+    # 0.5 = 30.5; constant-bound step 3 (time tested once per block)
+    "levy": (54.5, "Philox 21 (two words per variate) + CMS 30.5 + constant-bound step 3"),
+    # per accumulator: increment 12.4 (scale and drift folded in), add (packed)
+    # 0.5, clamp at 0 1, largest value so far (three-input) 0.5; time update per step
+    "race_no_bias_angle_4": (14.65, "normal 12.4 (six per Philox call) + add, clamp, maximum 2 "
+                                    "+ shared time update 1/4"),
+    # per accumulator: increment 12.4 (v dt + s sqrt(dt) N), the update
+    # x (1 - g dt + b dt) + S (-b dt) + increment as two packed FFMA 1, clamp 1,
+    # maximum 0.5; the sum S 3/4
+    "lca_no_bias_4": (15.65, "increment 12.4 + LCA update 1 + clamp, maximum 1.5 + sum 0.75"),
+    # per accumulator: increment 12.4, add (two of three packed) 2/3, maximum 2/3;
+    # time update per step 1/3
+    "racing_diffusion_3": (14.07, "increment 12.4 + add, maximum 1.33 + shared time update 1/3"),
 }
 E2E_WINDOWS = 5
 N_SM = 148
@@ -386,14 +384,14 @@ def run_ours(args, rank, world, local_rank):
                      "traffic": traffic, "traffic_unit": "DRAM bytes per launch (ncu)",
                      "algorithmic_bytes": total * 8,
                      "peak_basis": f"{N_SM} SMs x {LANES_PER_SM_CLK} lanes/clk x {f_max/1e6:.0f} MHz / "
-                                   f"{INSTR_PER_STEP:.0f} lane-instructions per accumulator-step",
+                                   f"{INSTR_PER_STEP:.1f} lane-instructions per accumulator-step",
                      "output_hbm_gbs": total * 8 / (ms_per_step / 1e3) / 1e9,
                      "hbm_peak_gbs": hbm_gbs, "hbm_peak_basis": hbm_basis,
                      "hbm_frac": total * 8 / (ms_per_step / 1e3) / 1e9 / hbm_gbs},
         "e2e": {"value": e2e_value, "unit": "trajectories/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
-        "gpu_launches": 2 * args.steps,
-        "e2e_launches": 2 * args.e2e_windows * args.steps,
+        "gpu_launches": 4 * args.steps,
+        "e2e_launches": 4 * args.e2e_windows * args.steps,
         "clocks": clocks,
     }
     return line, theta, n_samples

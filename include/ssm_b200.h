@@ -73,15 +73,15 @@ typedef struct ssm_launch {
     const int32_t *trial_order;
     const int64_t *order_offsets;
     /* Lanes per trajectory of the single-accumulator simulators (device RNG,
-     * constant / linear / Weibull boundary): 1, 2, 4, 8, 16 or 32; 0 = automatic,
+     * constant / linear / Weibull boundary): 1, 2, 4 or 8; 0 = automatic,
      * which is 1 for the ragged layout and otherwise chosen from the number
      * of trajectories against the grid's lanes (ssm_auto_lanes_per_walk).
-     * With W >= 8 the lanes of a group draw a walk's increments in parallel and
-     * share its tests: results are bit-identical to W = 1, and a launch
-     * with fewer trajectories than lanes ends sooner; chunk is 32 / W.  The
-     * library may take more lanes than asked for where the number of
-     * trajectories is small, and one lane (with the launch's last trajectories
-     * on several) for 2 and 4, which gained nothing over that. */
+     * With more than one the lanes of a group draw a walk's increments in
+     * parallel and share its tests: results are bit-identical to one, and a
+     * launch with fewer trajectories than lanes ends sooner.  The library takes
+     * the value as a statement of how short of trajectories the launch is: 8
+     * becomes 16 or 32 when the GPU holds all its walks that way, and 2 and 4
+     * become one lane with the launch's last trajectories on several. */
     int lanes_per_walk;
 } ssm_launch;
 

@@ -590,8 +590,8 @@ struct Launcher {
         }
         constexpr bool WIDE = WideOk<MODEL, NOISE, BOUND>::value;
         int W = (opt && opt->lanes_per_walk > 0) ? opt->lanes_per_walk : 1;
-        if (W != 1 && W != 2 && W != 4 && W != 8 && W != 16 && W != 32) {
-            set_error("lanes_per_walk must be 0 (automatic), 1, 2, 4, 8, 16 or 32");
+        if (W != 1 && W != 2 && W != 4 && W != 8) {
+            set_error("lanes_per_walk must be 0 (automatic), 1, 2, 4 or 8");
             return SSM_ERR_ARG;
         }
         if (W > 1 && !WIDE) {
@@ -599,7 +599,7 @@ struct Launcher {
             return SSM_ERR_ARG;
         }
         if (WIDE && call.total >= 0 && !(opt && opt->lanes_per_walk > 0)) W = auto_lanes_per_walk(call.total);
-        if (WIDE && W > 1 && W <= 8) W = effective_lanes(W, call.total, call.left != nullptr);
+        if (WIDE && W > 1) W = effective_lanes(W, call.total, call.left != nullptr);
         if (W > 1) return wide_launch(MODEL, BOUND, W, call, opt, st);
         SingleParams p = call;
         if (NOISE || BOUND == SSM_BOUND_TABLE) p.left = nullptr;

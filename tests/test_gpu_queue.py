@@ -66,7 +66,7 @@ def test_layouts_orders_and_shapes_agree(cuda, model, kind):
     order = np.random.default_rng(3).permutation(K).astype(np.int32)
     qoff = np.concatenate([[0], np.cumsum(NS[order])]).astype(np.int64)
     ot, qt = torch.from_numpy(order).cuda(), torch.from_numpy(qoff).cuda()
-    wide = [1] if model in ("levy_flexbound", "ddm_flex") or kind == _lib.BOUND_TABLE else [1, 2, 4, 8, 16, 32]
+    wide = [1] if model in ("levy_flexbound", "ddm_flex") or kind == _lib.BOUND_TABLE else [1, 2, 4, 8]
     for w in wide:
         for shape in ((32, 1, 32, 1), (64, 1, 256, 2), (256, 0, 64, 32)):
             lo = D.launch_opts(*shape[:3], refill_min=shape[3], lanes_per_walk=w)
@@ -75,6 +75,24 @@ def test_layouts_orders_and_shapes_agree(cuda, model, kind):
                 assert _lib.lib().ssm_check_status(D.ptr(out.workspace), D.stream_ptr()) == _lib.SSM_OK
                 for got, exp in zip(_bits(out), want):
                     np.testing.assert_array_equal(got, exp)
+
+
+@pytest.mark.parametrize("model,kind", [c for c in CASES if c[0] not in ("levy_flexbound", "ddm_flex")
+                                        and c[1] != _lib.BOUND_TABLE])
+def test_group_widths_agree(cuda, model, kind):
+    """A launch of known size takes 32, 16 or 8 lanes per walk (up to 24, 96 and more
+    walks per SM): the walks are those of one lane each."""
+    kw = _inputs(model, kind)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    run = lambda n, w: _bits(dev.simulate_single(model, n_trials=K, n_samples=n, max_t=3.0, seed=77,  # noqa: E731
+                                                 smooth_unif=True, want_steps=True, launch=D.launch_opts(lanes_per_walk=w),
+                                                 **kw))
+    want = run(100 * sms // K + 9, 1)
+    for walks in (1, 24 * sms, 24 * sms + 12, 96 * sms, 96 * sms + 24):
+        n = max(1, walks // K)
+        for w in (0, 8):
+            for got, exp in zip(run(n, w), want):
+                np.testing.assert_array_equal(got, exp[:n * K])
 
 
 @pytest.mark.parametrize("model,kind", CASES)
