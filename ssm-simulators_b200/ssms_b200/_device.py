@@ -83,6 +83,21 @@ def to_dev_f32_rows(xs: dict, n: int) -> dict:
     return out
 
 
+def upload(x: np.ndarray, stream: torch.cuda.Stream | None = None) -> torch.Tensor:
+    """A host array as a CUDA tensor for kernels on the current stream, without
+    waiting for the work queued there (a pageable copy does): through a
+    page-locked block that torch's caching host allocator recycles only after the
+    copy.  For another stream's kernels, and while a graph is captured, the plain copy."""
+    dev = require_cuda()
+    x = np.ascontiguousarray(x)
+    if stream is not None or x.size == 0 or torch.cuda.is_current_stream_capturing():
+        return torch.from_numpy(x).to(dev)
+    src = torch.from_numpy(x)
+    stage = torch.empty(src.shape, dtype=src.dtype, pin_memory=True)
+    stage.copy_(src)
+    return stage.to(dev, non_blocking=True)
+
+
 def workspace(nbytes: int, tag: int = 0, stream: torch.cuda.Stream | None = None) -> torch.Tensor:
     """A cached, 256-byte aligned device scratch buffer of at least ``nbytes``.
 

@@ -43,8 +43,8 @@ def bandwidth_silverman(sample: Iterable[float] = (0, 0, 0), std_cutoff: float =
     return np.power((4 / (3 * n)), 1 / 5) * std
 
 
-def _i64(x, dev):
-    return torch.as_tensor(np.asarray(x, dtype=np.int64)).to(dev) if not isinstance(x, torch.Tensor) else x.to(dev, torch.int64).contiguous()
+def _i64(x, dev, stream=None):
+    return D.upload(np.asarray(x, np.int64), stream) if not isinstance(x, torch.Tensor) else x.to(dev, torch.int64).contiguous()
 
 
 class KdeBatch:
@@ -55,20 +55,20 @@ class KdeBatch:
         dev = D.require_cuda()
         self.choice_values = np.unique(np.asarray(possible_choices)).astype(np.int32)
         self.nc = int(self.choice_values.shape[0])
-        self.sample_offsets = _i64(sample_offsets, dev)
+        self.sample_offsets = _i64(sample_offsets, dev, stream)
         self.n_sets = int(self.sample_offsets.numel() - 1)
         G = self.n_sets * self.nc
         total = int(rts.numel())
         self.rts = rts.to(dev, torch.float32).contiguous().reshape(-1)
         self.choices = choices.to(dev, torch.int32).contiguous().reshape(-1)
-        self.cvals = torch.as_tensor(self.choice_values).to(dev)
+        self.cvals = D.upload(self.choice_values, stream)
         self.displace = None
         self.displaced_logs = None
         if displace is not None:
             dsp = np.asarray(displace, dtype=np.float64).reshape(-1)
             if dsp.shape[0] < self.n_sets:
                 raise ValueError("displace needs one value per set")
-            self.displace = torch.from_numpy(np.ascontiguousarray(dsp)).to(dev)
+            self.displace = D.upload(dsp, stream)
             self.displaced_logs = torch.empty(max(total, 1), dtype=torch.float64, device=dev)
         self.count_all = torch.empty(G, dtype=torch.int64, device=dev)
         self.n_valid = torch.empty(G, dtype=torch.int64, device=dev)
@@ -91,7 +91,7 @@ class KdeBatch:
         """Log-likelihoods of queries sorted by group (query_offsets: [G + 1])."""
         dev = D.require_cuda()
         qoff_host = None if isinstance(query_offsets, torch.Tensor) else np.asarray(query_offsets, np.int64)
-        qoff = _i64(query_offsets, dev)
+        qoff = _i64(query_offsets, dev, self.stream)
         q = query_rt.to(dev, torch.float64).contiguous().reshape(-1)
         n_q = int(qoff_host[-1]) if qoff_host is not None else int(qoff[-1].item())
         if n_q > q.numel():
@@ -110,8 +110,8 @@ class KdeBatch:
                unif_hi: float | None = None) -> torch.Tensor:
         """Per group: n_kde[g] KDE draws then U(unif_lo, unif_hi) rts up to out_offsets[g+1]."""
         dev = D.require_cuda()
-        ooff = _i64(out_offsets, dev)
-        nk = _i64(n_kde, dev)
+        ooff = _i64(out_offsets, dev, self.stream)
+        nk = _i64(n_kde, dev, self.stream)
         total = int(ooff[-1].item())
         out = torch.empty(max(total, 1), dtype=torch.float64, device=dev)
         _lib.check(_lib.lib().ssm_kde_sample(
