@@ -91,6 +91,12 @@ __device__ __forceinline__ Slice set_slice(const int64_t *soff, int64_t n_sets) 
     return s;
 }
 
+// A barrier of the set's CTAs.
+__device__ __forceinline__ void sync_set(const Slice &s) {
+    if (s.J > 1) cooperative_groups::this_cluster().sync();
+    else __syncthreads();
+}
+
 // f(rt, choice) for the samples [lo, hi) in no particular order: 16-byte loads
 // where both arrays allow them (same offset from a 16-byte boundary), scalar
 // loads at the ragged ends and otherwise.
@@ -201,20 +207,69 @@ __global__ void k_scan_i64(const int64_t *in, int64_t n, int64_t *out) {
     if (threadIdx.x == 0) out[n] = carry;
 }
 
-__device__ __forceinline__ double block_sum_f64(double v, double *red) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) red[warp] = v;
+// Sums over the points of the set's groups by its whole cluster: f(c, x) over group
+// c's points (or displaced bandwidth inputs), the total of choice c to out[c].  The
+// points' rows of 32 go round KDE_PLACES places, and the cluster's warps share the
+// places, K = KDE_PLACES / (8 J) to a warp with their loads in flight together.  A
+// place's sum and the sum of the places are the same additions whatever J is, so
+// a set's moments have the same bits in any call.
+constexpr int KDE_PLACES = 64;  // the warps of the largest cluster
+template <int NC, int K, class F>
+__device__ __forceinline__ void sum_places(const KdeFit &a, const Slice &sl, double *place, F f) {
+    constexpr int WARPS = KDE_PLACES / K;
+    const int lane = threadIdx.x & 31, gw = (int)(sl.rank * 8 + (threadIdx.x >> 5));
+    for (int c = 0; c < a.nc; ++c) {
+        const int64_t g = sl.set * a.nc + c, lo = a.poff[g], n = a.poff[g + 1] - lo;
+        const int first = (gw - c) & (WARPS - 1);  // small groups of different choices go to different warps
+        if (32 * first >= n) continue;
+        const double *bw = a.bwvals ? a.bwvals + lo : nullptr;
+        const float *pt = a.points + lo;
+        double t[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) t[k] = 0.0;
+        for (int64_t i = 32 * first + lane; i < n; i += 32 * KDE_PLACES) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const int64_t at = i + 32 * WARPS * k;
+                if (at < n) t[k] += f(c, bw ? __ldcg(bw + at) : (double)__ldcg(pt + at));
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) t[k] += __shfl_down_sync(0xffffffffu, t[k], o);
+        }
+        if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) place[c * KDE_PLACES + first + WARPS * k] = t[k];
+        }
+    }
+}
+// (place: NC * KDE_PLACES values of shared memory that no other CTA of the cluster
+// still reads; ends with a barrier of the CTA alone)
+template <int NC, class F>
+__device__ __forceinline__ void sum_points(const KdeFit &a, const Slice &sl, double *place, double *out, F f) {
+    switch (sl.J) {
+        case 1: sum_places<NC, 8>(a, sl, place, f); break;
+        case 2: sum_places<NC, 4>(a, sl, place, f); break;
+        case 4: sum_places<NC, 2>(a, sl, place, f); break;
+        default: sum_places<NC, 1>(a, sl, place, f); break;
+    }
+    sync_set(sl);
+    const int lane = threadIdx.x & 31;
+    for (int c = threadIdx.x >> 5; c < a.nc; c += 8) {
+        const int64_t n = a.poff[sl.set * a.nc + c + 1] - a.poff[sl.set * a.nc + c];
+        double t = 0.0;
+#pragma unroll
+        for (int v = lane; v < KDE_PLACES; v += 32)
+            if (32 * v < n)
+                t += cooperative_groups::this_cluster().map_shared_rank(
+                    place, ((v + c) & (8 * sl.J - 1)) >> 3)[c * KDE_PLACES + v];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) out[c] = t;
+    }
     __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    __syncthreads();
-    if (threadIdx.x == 0) red[0] = t;
-    __syncthreads();
-    const double r = red[0];
-    __syncthreads();
-    return r;
 }
 
 // Stable per-choice compaction of log(rt - shift) into the group regions, then
@@ -225,19 +280,22 @@ __device__ __forceinline__ double block_sum_f64(double v, double *red) {
 // lower ranks' counts; then it walks the slice in chunks of 1 024 samples, four
 // consecutive ones per thread.  Ranks inside a chunk come from a warp scan of
 // byte-packed counts (four choices in one word, at most 128 each) and the warps'
-// totals, one barrier per chunk.  Sums of the log-rts are taken on the way;
-// the squared deviations from the mean are a second pass over the group's
-// points, still in L2, shared by the cluster.  What remains is the float64
-// logarithm of every sample.  One CTA per set with a barrier pair per 256 samples
-// and the moments in a kernel of their own had taken 87 + 13 us for 128 sets of
-// 20 000 samples and 348 + 45 us for 256 of 50 000.
+// totals, one barrier per chunk.  Mean and squared deviations are two passes over
+// the group's points, still in L2, shared by the cluster (sum_points).  What
+// remains is the float64 logarithm of every sample.  One CTA per set with a barrier
+// pair per 256 samples and the moments in a kernel of their own had taken 87 + 13 us
+// for 128 sets of 20 000 samples and 348 + 45 us for 256 of 50 000.  The whole fit, us,
+// with the mean's sums taken on the way (in an order that followed the cluster's size)
+// and now: those two 88 and 236, now 84 and 233; two million samples in one set 995,
+// now 818; 1 000 sets of 100 000 1 328, now 1 405; 5 000 sets of 200 122, now 134; four
+// choices 1 934, now 1 798, and 192, now 169.
 template <int NC>
-__global__ void __launch_bounds__(256) k_kde_scatter(const KdeFit a) {
+__global__ void __launch_bounds__(256, NC == 2 ? 6 : NC == 4 ? 5 : 3) k_kde_scatter(const KdeFit a) {
     namespace cg = cooperative_groups;
     constexpr int W = 8, NW = (NC + 3) / 4;
     __shared__ unsigned int tot[NC];
     __shared__ __align__(16) unsigned int wtot[2][NW][W];
-    __shared__ double red[32], csum[NC], css[NC];
+    __shared__ double place[2][NC * KDE_PLACES], mean[NC], dev[NC];
     cg::cluster_group cl = cg::this_cluster();
     const Slice sl = set_slice(a.soff, a.n_sets);
     const ChoiceSet<NC> cs(a.cvals, a.nc);
@@ -273,10 +331,6 @@ __global__ void __launch_bounds__(256) k_kde_scatter(const KdeFit a) {
             for (int c = 0; c < NC; ++c) base[c] += t[c];
         }
     }
-    double s1[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) s1[c] = 0.0;
-
     const bool vec = ((((uintptr_t)a.rts ^ (uintptr_t)a.choices) & 15u) == 0);
     const int64_t start = sl.lo - (int64_t)(((uintptr_t)(a.rts + sl.lo) >> 2) & 3);  // 16-byte boundary at or before lo
     int buf = 0;
@@ -356,44 +410,25 @@ __global__ void __launch_bounds__(256) k_kde_scatter(const KdeFit a) {
             const float r = a.shift ? __double2float_rn((double)rt[q] - sh) : rt[q];
             const float x = __double2float_rn(log((double)r));
             a.points[at] = x;
-            double m = (double)x;
-            if (a.bwvals) {
-                m = log(exp((double)__double2float_rn(log((double)rt[q]))) - sh);
-                a.bwvals[at] = m;
-            }
-#pragma unroll
-            for (int c = 0; c < NC; ++c)
-                if (ci[q] == c) s1[c] += m;
+            if (a.bwvals) a.bwvals[at] = log(exp((double)__double2float_rn(log((double)rt[q]))) - sh);
         }
     }
-    // mean of each group: the ranks' sums in rank order
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-        if (c < a.nc) {
-            const double t = block_sum_f64(s1[c], red);
-            if (threadIdx.x == 0) csum[c] = t;
-        }
-    cl.sync();  // also orders the cluster's point writes before the reads below
-    for (int c = 0; c < a.nc; ++c) {
-        const int64_t g = sl.set * a.nc + c, lo = a.poff[g], n = a.poff[g + 1] - lo;
-        double mean = 0.0;
-        for (unsigned j = 0; j < sl.J; ++j) mean += cl.map_shared_rank(csum, j)[c];
-        mean /= (double)(n > 0 ? n : 1);
-        double ss = 0.0;
-        for (int64_t i = (int64_t)sl.rank * blockDim.x + threadIdx.x; i < n; i += (int64_t)sl.J * blockDim.x) {
-            const double d = (a.bwvals ? __ldcg(a.bwvals + lo + i) : (double)__ldcg(a.points + lo + i)) - mean;
-            ss += d * d;
-        }
-        const double t = block_sum_f64(ss, red);
-        if (threadIdx.x == 0) css[c] = t;
+    sync_set(sl);  // orders the cluster's point writes before the reads below
+    sum_points<NC>(a, sl, place[0], mean, [](int, double x) { return x; });
+    if ((int)threadIdx.x < a.nc) {
+        const int64_t g = sl.set * a.nc + threadIdx.x, n = a.poff[g + 1] - a.poff[g];
+        mean[threadIdx.x] /= (double)(n > 0 ? n : 1);
     }
-    cl.sync();
+    __syncthreads();
+    sum_points<NC>(a, sl, place[1], dev, [&](int c, double x) {
+        const double d = x - mean[c];
+        return d * d;
+    });
     if (sl.rank == 0 && threadIdx.x < a.nc) {
         const int c = threadIdx.x;
         const int64_t g = sl.set * a.nc + c, n = a.poff[g + 1] - a.poff[g];
         const int64_t N = a.soff[sl.set + 1] - a.soff[sl.set];
-        double ss = 0.0;
-        for (unsigned j = 0; j < sl.J; ++j) ss += cl.map_shared_rank(css, j)[c];
+        const double ss = dev[c];
         const double var = ss / (double)(n > 0 ? n : 1);
         const double p = (N > 0) ? (double)a.count_all[g] / (double)N : 0.0;
         a.prop[g] = p;
@@ -408,7 +443,7 @@ __global__ void __launch_bounds__(256) k_kde_scatter(const KdeFit a) {
             a.lognorm[g] = log(p) - log((double)n) - log(h) - 0.5 * KDE_LOG_2PI;
         }
     }
-    cl.sync();  // rank 0 has read the others' sums
+    sync_set(sl);  // the others have read this CTA's places
 }
 
 struct KdeEval {
