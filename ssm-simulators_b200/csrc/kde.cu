@@ -123,7 +123,8 @@ __device__ __forceinline__ void for_each_sample(const float *rts, const int32_t 
 }
 
 // Samples per choice, with and without omissions.  Bound by reading 8 bytes a
-// sample: the counts stay in registers (one compare-and-add per choice), are
+// sample: the counts stay in registers (one compare-and-add per choice; 32 bits
+// hold a warp's share of a slice of 2^35 samples, more than the memory does), are
 // summed over the warp by one reduction each, and the cluster's CTAs meet in
 // rank 0.  Two 64-bit shared counters per choice, which every lane hit, had
 // serialised the whole pass: 128 sets of 20 000 samples 831 us, 256 of 50 000
@@ -131,10 +132,10 @@ __device__ __forceinline__ void for_each_sample(const float *rts, const int32_t 
 template <int NC>
 __global__ void __launch_bounds__(256) k_kde_count(const KdeFit a) {
     namespace cg = cooperative_groups;
-    __shared__ unsigned int tot[2 * NC];
+    __shared__ unsigned long long tot[2 * NC];
     const Slice sl = set_slice(a.soff, a.n_sets);
     const ChoiceSet<NC> cs(a.cvals, a.nc);
-    if (threadIdx.x < 2 * NC) tot[threadIdx.x] = 0u;
+    if (threadIdx.x < 2 * NC) tot[threadIdx.x] = 0ull;
     __syncthreads();
     unsigned int all[NC], val[NC];
 #pragma unroll
@@ -153,8 +154,8 @@ __global__ void __launch_bounds__(256) k_kde_count(const KdeFit a) {
     for (int c = 0; c < NC; ++c) {
         const unsigned int x = __reduce_add_sync(0xffffffffu, all[c]), y = __reduce_add_sync(0xffffffffu, val[c]);
         if (lane == 0) {
-            atomicAdd(&tot[c], x);
-            atomicAdd(&tot[NC + c], y);
+            atomicAdd(&tot[c], (unsigned long long)x);
+            atomicAdd(&tot[NC + c], (unsigned long long)y);
         }
     }
     cg::cluster_group cl = cg::this_cluster();
@@ -162,9 +163,9 @@ __global__ void __launch_bounds__(256) k_kde_count(const KdeFit a) {
     if (sl.rank == 0 && threadIdx.x < a.nc) {
         int64_t x = 0, y = 0;
         for (unsigned j = 0; j < sl.J; ++j) {
-            const unsigned int *t = cl.map_shared_rank(tot, j);
-            x += t[threadIdx.x];
-            y += t[NC + threadIdx.x];
+            const unsigned long long *t = cl.map_shared_rank(tot, j);
+            x += (int64_t)t[threadIdx.x];
+            y += (int64_t)t[NC + threadIdx.x];
         }
         a.count_all[sl.set * a.nc + threadIdx.x] = x;
         a.n_valid[sl.set * a.nc + threadIdx.x] = y;
@@ -293,7 +294,7 @@ template <int NC>
 __global__ void __launch_bounds__(256, NC == 2 ? 6 : NC == 4 ? 5 : 3) k_kde_scatter(const KdeFit a) {
     namespace cg = cooperative_groups;
     constexpr int W = 8, NW = (NC + 3) / 4;
-    __shared__ unsigned int tot[NC];
+    __shared__ unsigned long long tot[NC];
     __shared__ __align__(16) unsigned int wtot[2][NW][W];
     __shared__ double place[2][NC * KDE_PLACES], mean[NC], dev[NC];
     cg::cluster_group cl = cg::this_cluster();
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(256, NC == 2 ? 6 : NC == 4 ? 5 : 3) k_kde_scat
     // this slice's counts, then the position of its first sample of each choice
     int64_t base[NC];
     {
-        if (threadIdx.x < NC) tot[threadIdx.x] = 0u;
+        if (threadIdx.x < NC) tot[threadIdx.x] = 0ull;
         __syncthreads();
         if (sl.J > 1) {
             unsigned int val[NC];
@@ -319,16 +320,16 @@ __global__ void __launch_bounds__(256, NC == 2 ? 6 : NC == 4 ? 5 : 3) k_kde_scat
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 const unsigned int y = __reduce_add_sync(0xffffffffu, val[c]);
-                if (lane == 0) atomicAdd(&tot[c], y);
+                if (lane == 0) atomicAdd(&tot[c], (unsigned long long)y);
             }
         }
         cl.sync();
 #pragma unroll
         for (int c = 0; c < NC; ++c) base[c] = (c < a.nc) ? a.poff[sl.set * a.nc + c] : 0;
         for (unsigned j = 0; j < sl.rank; ++j) {
-            const unsigned int *t = cl.map_shared_rank(tot, j);
+            const unsigned long long *t = cl.map_shared_rank(tot, j);
 #pragma unroll
-            for (int c = 0; c < NC; ++c) base[c] += t[c];
+            for (int c = 0; c < NC; ++c) base[c] += (int64_t)t[c];
         }
     }
     const bool vec = ((((uintptr_t)a.rts ^ (uintptr_t)a.choices) & 15u) == 0);
@@ -955,7 +956,9 @@ __device__ __forceinline__ int np_hist_index(float rt, double max_t, double step
 
 // One pass over a set's samples by its cluster: counts in registers, the
 // histograms as 32-bit shared counters per CTA (equal bins of a warp are added
-// up by the hardware), added over the cluster at the end.  A histogram with half
+// up by the hardware), added over the cluster at the end.  A slice of more than
+// 2^31 samples is counted in parts, after each of which the counters' top bits move
+// to a byte of their own (the memory holds less than 2^35 samples).  A histogram with half
 // the bins of the other is its pairwise sum (its edges are every second one,
 // exactly: the steps differ by a power of two).  64-bit shared counters hit by
 // every lane and two float64 divisions per sample: 256 sets of 50 000 samples
@@ -963,8 +966,8 @@ __device__ __forceinline__ int np_hist_index(float rt, double max_t, double step
 template <int NC>
 __global__ void __launch_bounds__(256) k_set_summary(const SetSummary a) {
     namespace cg = cooperative_groups;
-    extern __shared__ unsigned int sh[];  // [nc * (nb_a + nb_b)] histogram counters
-    __shared__ unsigned int cnt[NC + 2];  // choices, no-go, omissions
+    extern __shared__ unsigned int sh[];  // [nc * (nb_a + nb_b)] histogram counters, then a byte of 2^31s each
+    __shared__ unsigned long long cnt[NC + 2];  // choices, no-go, omissions
     cg::cluster_group cl = cg::this_cluster();
     const Slice sl = set_slice(a.soff, a.n_sets);
     const ChoiceSet<NC> cs(a.cvals, a.nc);
@@ -973,17 +976,23 @@ __global__ void __launch_bounds__(256) k_set_summary(const SetSummary a) {
     const double step_a = a.max_t / (double)a.nb_a, step_b = a.max_t / (double)a.nb_b;
     const float inv_a = (float)(1.0 / step_a), inv_b = (float)(1.0 / step_b);
     unsigned int *hb = sh + a.nc * a.nb_a;
+    unsigned char *top = reinterpret_cast<unsigned char *>(sh + H);
+    constexpr int64_t PART = (int64_t)1 << 31;
+    const bool parts = sl.hi - sl.lo > PART;
     int32_t max_choice = cs.v[0];
 #pragma unroll
     for (int c = 1; c < NC; ++c)
         if (c < a.nc) max_choice = max(max_choice, cs.v[c]);
-    for (int i = threadIdx.x; i < H; i += blockDim.x) sh[i] = 0u;
-    if (threadIdx.x < NC + 2) cnt[threadIdx.x] = 0u;
+    for (int i = threadIdx.x; i < H; i += blockDim.x) {
+        sh[i] = 0u;
+        top[i] = 0;
+    }
+    if (threadIdx.x < NC + 2) cnt[threadIdx.x] = 0ull;
     __syncthreads();
     unsigned int n[NC], nogo = 0u, omit = 0u;
 #pragma unroll
     for (int c = 0; c < NC; ++c) n[c] = 0u;
-    for_each_sample(a.rts, a.choices, sl.lo, sl.hi, [&](float rt, int32_t ch) {
+    const auto sample = [&](float rt, int32_t ch) {
         const bool omitted = (rt == -999.f);
         omit += (ch == -999);
         nogo += (ch != max_choice || omitted);
@@ -997,30 +1006,42 @@ __global__ void __launch_bounds__(256) k_set_summary(const SetSummary a) {
             const int ia = np_hist_index(rt, a.max_t, step_a, inv_a, a.nb_a);
             if (ia >= 0) atomicAdd(&sh[c * a.nb_a + ia], 1u);
         }
-    });
+    };
+    for (int64_t lo = sl.lo; lo < sl.hi; lo += PART) {
+        for_each_sample(a.rts, a.choices, lo, min(lo + PART, sl.hi), sample);
+        if (parts) {
+            __syncthreads();
+            for (int i = threadIdx.x; i < H; i += blockDim.x) {
+                top[i] += (unsigned char)(sh[i] >> 31);
+                sh[i] &= 0x7fffffffu;
+            }
+            __syncthreads();
+        }
+    }
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         const unsigned int x = __reduce_add_sync(0xffffffffu, n[c]);
-        if (lane == 0 && c < a.nc) atomicAdd(&cnt[c], x);
+        if (lane == 0 && c < a.nc) atomicAdd(&cnt[c], (unsigned long long)x);
     }
     nogo = __reduce_add_sync(0xffffffffu, nogo);
     omit = __reduce_add_sync(0xffffffffu, omit);
     if (lane == 0) {
-        atomicAdd(&cnt[NC], nogo);
-        atomicAdd(&cnt[NC + 1], omit);
+        atomicAdd(&cnt[NC], (unsigned long long)nogo);
+        atomicAdd(&cnt[NC + 1], (unsigned long long)omit);
     }
     if (pairs) {
         __syncthreads();
         for (int i = threadIdx.x; i < a.nc * a.nb_a; i += blockDim.x) {
-            const int c = i / a.nb_a, k = i - c * a.nb_a;
-            sh[i] = hb[c * a.nb_b + 2 * k] + hb[c * a.nb_b + 2 * k + 1];
+            const int c = i / a.nb_a, k = i - c * a.nb_a, j = c * a.nb_b + 2 * k;
+            sh[i] = hb[j] + hb[j + 1];  // both below 2^31
+            top[i] = top[a.nc * a.nb_a + j] + top[a.nc * a.nb_a + j + 1];
         }
     }
     cl.sync();
     if (sl.rank == 0 && threadIdx.x < NC + 2) {
         int64_t x = 0;
-        for (unsigned j = 0; j < sl.J; ++j) x += cl.map_shared_rank(cnt, j)[threadIdx.x];
+        for (unsigned j = 0; j < sl.J; ++j) x += (int64_t)cl.map_shared_rank(cnt, j)[threadIdx.x];
         if ((int)threadIdx.x < a.nc) a.counts[sl.set * a.nc + threadIdx.x] = x;
         if (threadIdx.x == NC) a.nogo[sl.set] = x;
         if (threadIdx.x == NC + 1) a.omit[sl.set] = x;
@@ -1028,7 +1049,8 @@ __global__ void __launch_bounds__(256) k_set_summary(const SetSummary a) {
     // layout [S, nb, nc] like the pipeline's binned_128 / binned_256 arrays; the ranks share the bins
     for (int i = (int)sl.rank * (int)blockDim.x + threadIdx.x; i < H; i += (int)(sl.J * blockDim.x)) {
         int64_t x = 0;
-        for (unsigned j = 0; j < sl.J; ++j) x += cl.map_shared_rank(sh, j)[i];
+        for (unsigned j = 0; j < sl.J; ++j)
+            x += (int64_t)cl.map_shared_rank(sh, j)[i] + ((int64_t)cl.map_shared_rank(top, j)[i] << 31);
         if (i < a.nc * a.nb_a) {
             const int c = i / a.nb_a, b = i % a.nb_a;
             a.hist_a[(sl.set * a.nb_a + b) * a.nc + c] = (float)x;
@@ -1054,6 +1076,7 @@ static int launch_per_set(K kernel, const A &args, int64_t n_sets, size_t smem, 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n_sets * J));
     cfg.blockDim = dim3(256);
+    if (smem > 48 * 1024) SSM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -1096,7 +1119,7 @@ int ssm_set_summary(const float *rts, const int32_t *choices, int64_t n_sets,
     a.rts = rts; a.choices = choices; a.soff = sample_offsets; a.cvals = choice_values;
     a.nc = n_choices; a.max_t = max_t; a.counts = choice_counts; a.nogo = nogo_counts;
     a.omit = omission_counts; a.nb_a = nbins_a; a.nb_b = nbins_b; a.hist_a = hist_a; a.hist_b = hist_b;
-    const size_t smem = (size_t)n_choices * (nbins_a + nbins_b) * sizeof(unsigned int);
+    const size_t smem = (size_t)n_choices * (nbins_a + nbins_b) * (sizeof(unsigned int) + 1);
     SSM_REQUIRE(n_sets < (int64_t)1 << 28, "too many sets for one launch");
     cudaStream_t st = (cudaStream_t)stream;
     if (n_choices <= 2) return launch_per_set(k_set_summary<2>, a, n_sets, smem, st);
