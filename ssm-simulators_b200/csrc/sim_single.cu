@@ -359,6 +359,7 @@ __device__ __forceinline__ void finalize(const SingleParams &p, const Lane &L) {
 template <int MODEL, int BOUND, bool NOISE>
 __global__ void __launch_bounds__(256, 3) k_single(const __grid_constant__ SingleParams p) {
     constexpr int BLK = Blk<MODEL, BOUND>::value;
+    static_assert(BLK % 2 == 0, "walks are handed over at even steps (TimeSteps, sim_wide.cu)");
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;

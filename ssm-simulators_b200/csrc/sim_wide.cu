@@ -37,12 +37,19 @@ template <int MODEL> struct Seg { static constexpr int value = (MODEL == M_LEVY)
 constexpr int SEG_STRIDE = 20;  // floats between segments in shared memory: 16-byte rows, no bank conflicts
 constexpr int WIDE_WARPS = 8;
 
-// The float32 time accumulator after n more additions of dt.  Round to nearest
-// moves a multiple of the binade's ulp u by dt rounded to a multiple of u; only
-// a tie depends on the last bit, and its result is even, so from the second
-// addition on the amount is the same.  next = RN(t + dt) and inc = RN(next + dt) - next
-// are exact values, and after n >= 1 additions the accumulator is next + (n - 1) inc
-// exactly, as long as that stays in next's binade.
+// The float32 time accumulator t = dt + dt + ... (an even number of additions) after n
+// more of them.  Inside one binade, of ulp u, an addition moves it by dt rounded to a
+// multiple of u, the same every time unless dt is an odd multiple of u / 2: then
+// each addition is a tie with an even result, so the amount is the same from an
+// even accumulator on.  next = RN(t + dt) is even in that case: if t lies in the same
+// binade, it is such a result; if t lies below, all additions so far were exact (dt
+// is a multiple of every smaller ulp), t + dt = (k + 1) dt after k of them, and with
+// k even this is an odd multiple of u / 2, a tie again.  (With k odd it could be exact
+// and odd, and the additions after the first would differ: k = 1 049, dt =
+// 15979 / 2^24.)  So next and inc = RN(next + dt) - next are exact values, and after
+// n >= 1 additions the accumulator is next + (n - 1) inc exactly, as long as that
+// stays in next's binade.  Walks start at step 0, are handed over after whole blocks of
+// the one-lane mode and advance by whole blocks here: all even (asserted).
 struct TimeSteps {
     float t, next, inc;
     __device__ __forceinline__ TimeSteps(float t0, float dt) : t(t0) {
@@ -228,6 +235,7 @@ template <int MODEL, int BOUND, int W>
 __global__ void __launch_bounds__(32 * WIDE_WARPS, 2) k_wide(const __grid_constant__ SingleParams p) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int SEG = Seg<MODEL>::value, BLK = SEG * W;
+    static_assert(BLK % 2 == 0, "TimeSteps: a block starts at an even step");
     __shared__ __align__(16) float shared[WIDE_WARPS][32 * SEG_STRIDE];
     if constexpr (WideOk<MODEL, false, BOUND>::value) {
         if (p.traj != nullptr && blockIdx.x == gridDim.x - 1) {
