@@ -347,6 +347,9 @@ __device__ __forceinline__ bool advance_window(const RaceParams &p, RaceLane<NP>
                                                const float *pre) {
     constexpr int WIN = RaceWin<NP>::value;
     constexpr bool LCA = (FAM == FAM_LCA), ONE_TEST = (BOUND == SSM_BOUND_CONSTANT || BOUND == SSM_BOUND_LINEAR);
+    // (a walk of the other families ends above its bound, which is what the test of
+    // each step for the other bounds looks for)
+    static_assert(FAM != FAM_RDM || BOUND == SSM_BOUND_CONSTANT, "racing diffusion ends at or above a constant bound");
     if (window_clear<NP, FAM>(p, L, h, WIN)) {
         // accumulators 0 and 1 in x01, 2 and 3 in x23 (2 alone: its upper half is idle)
         uint64_t xp[(NP + 1) / 2];
@@ -846,10 +849,16 @@ static int race_launch(const RaceParams &p, const ssm_launch *opt, cudaStream_t 
     return SSM_OK;
 }
 
+// Racing diffusion has a constant bound (ssm_racing_diffusion takes no other); the
+// kernels of its other forms are not built.
 template <int NP, int FAM>
 static int race_dispatch_bound(int bound, bool noise, const RaceParams &p, const ssm_launch *opt,
                                cudaStream_t st) {
-    if (noise) {  // exact mode: any boundary shape arrives as a host table or in closed form
+    if constexpr (FAM == FAM_RDM) {
+        SSM_REQUIRE(bound == SSM_BOUND_CONSTANT, "racing diffusion has a constant boundary");
+        return noise ? race_launch<NP, FAM, SSM_BOUND_CONSTANT, true>(p, opt, st)
+                     : race_launch<NP, FAM, SSM_BOUND_CONSTANT, false>(p, opt, st);
+    } else if (noise) {  // exact mode: any boundary shape arrives as a host table or in closed form
         switch (bound) {
             case SSM_BOUND_TABLE: return race_launch<NP, FAM, SSM_BOUND_TABLE, true>(p, opt, st);
             case SSM_BOUND_CONSTANT: return race_launch<NP, FAM, SSM_BOUND_CONSTANT, true>(p, opt, st);
@@ -858,16 +867,17 @@ static int race_dispatch_bound(int bound, bool noise, const RaceParams &p, const
         }
         set_error("noise injection supports table, constant and linear boundaries");
         return SSM_ERR_ARG;
+    } else {
+        switch (bound) {
+            case SSM_BOUND_TABLE: return race_launch<NP, FAM, SSM_BOUND_TABLE, false>(p, opt, st);
+            case SSM_BOUND_CONSTANT: return race_launch<NP, FAM, SSM_BOUND_CONSTANT, false>(p, opt, st);
+            case SSM_BOUND_LINEAR: return race_launch<NP, FAM, SSM_BOUND_LINEAR, false>(p, opt, st);
+            case SSM_BOUND_WEIBULL: return race_launch<NP, FAM, SSM_BOUND_WEIBULL, false>(p, opt, st);
+            default: break;
+        }
+        set_error("unknown boundary kind %d", bound);
+        return SSM_ERR_ARG;
     }
-    switch (bound) {
-        case SSM_BOUND_TABLE: return race_launch<NP, FAM, SSM_BOUND_TABLE, false>(p, opt, st);
-        case SSM_BOUND_CONSTANT: return race_launch<NP, FAM, SSM_BOUND_CONSTANT, false>(p, opt, st);
-        case SSM_BOUND_LINEAR: return race_launch<NP, FAM, SSM_BOUND_LINEAR, false>(p, opt, st);
-        case SSM_BOUND_WEIBULL: return race_launch<NP, FAM, SSM_BOUND_WEIBULL, false>(p, opt, st);
-        default: break;
-    }
-    set_error("unknown boundary kind %d", bound);
-    return SSM_ERR_ARG;
 }
 
 template <int FAM>
