@@ -212,14 +212,11 @@ __device__ __forceinline__ bool window_clear(const RaceParams &p, const RaceLane
 // failed before the step (the walk is over).  With PRE the step's increments
 // v_j dt + sq_j N(0,1) come from pre[j * PSTRIDE] (draw_window); ctr still
 // counts the steps.
-// CHECKED false skips the step-cap check and the time test, for a window the
-// caller has shown both to pass for (window_clear).
-template <int NP, int FAM, int BOUND, bool NOISE, bool RECORD, bool PRE = false, bool CHECKED = true,
-          int PSTRIDE = 1>
+template <int NP, int FAM, int BOUND, bool NOISE, bool RECORD, bool PRE = false, int PSTRIDE = 1>
 __device__ __forceinline__ bool race_step(const RaceParams &p, RaceLane<NP> &L, const RaceHead &h,
                                           const float *v, const float *sq, int np, uint32_t &ctr,
                                           const float *pre = nullptr) {
-    if (CHECKED && L.ixf >= h.capf) {
+    if (L.ixf >= h.capf) {
         raise_error(p.hdr, SSM_ERR_DEVICE, (int)L.w);
         return false;
     }
@@ -231,7 +228,7 @@ __device__ __forceinline__ bool race_step(const RaceParams &p, RaceLane<NP> &L, 
             if (j < np) finished |= (L.x[j] > bnd);
     }
     constexpr bool LCA = (FAM == FAM_LCA);
-    const bool in_time = !CHECKED || (LCA ? (L.tpd <= (double)h.dl_tmp) : (L.tp <= h.dl_tmp));
+    const bool in_time = LCA ? (L.tpd <= (double)h.dl_tmp) : (L.tp <= h.dl_tmp);
     if (finished || !in_time) return false;
     float gsn[NP];
     if (NOISE) {
@@ -436,7 +433,7 @@ __device__ __forceinline__ bool advance_window(const RaceParams &p, RaceLane<NP>
     uint32_t unused = 0;
 #pragma unroll
     for (int s = 0; s < WIN; ++s)
-        if (live) live = race_step<NP, FAM, BOUND, false, false, true, true, WIN>(p, L, h, nullptr, nullptr, NP, unused, pre + s);
+        if (live) live = race_step<NP, FAM, BOUND, false, false, true, WIN>(p, L, h, nullptr, nullptr, NP, unused, pre + s);
     return live;
 }
 
@@ -811,7 +808,7 @@ __global__ void k_race_record(const __grid_constant__ RaceParams p) {
             ctr += 4;
             uint32_t unused = 0;
             for (int s = 0; s < WIN && live; ++s)
-                live = race_step<NP, FAM, BOUND, NOISE, true, true, true, WIN>(p, L, h, vr, sr, np, unused, nrm + s);
+                live = race_step<NP, FAM, BOUND, NOISE, true, true, WIN>(p, L, h, vr, sr, np, unused, nrm + s);
         }
     } else {
         while (race_step<NP, FAM, BOUND, NOISE, true>(p, L, h, vr, sr, np, ctr)) {
