@@ -1073,6 +1073,7 @@ static unsigned ctas_per_set(int64_t n_sets) {
 template <class K, class A>
 static int launch_per_set(K kernel, const A &args, int64_t n_sets, size_t smem, cudaStream_t st) {
     const unsigned J = ctas_per_set(n_sets);
+    SSM_REQUIRE(n_sets <= (int64_t)INT32_MAX / J, "too many sets for one launch");  // the grid's limit
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n_sets * J));
     cfg.blockDim = dim3(256);
@@ -1120,7 +1121,6 @@ int ssm_set_summary(const float *rts, const int32_t *choices, int64_t n_sets,
     a.nc = n_choices; a.max_t = max_t; a.counts = choice_counts; a.nogo = nogo_counts;
     a.omit = omission_counts; a.nb_a = nbins_a; a.nb_b = nbins_b; a.hist_a = hist_a; a.hist_b = hist_b;
     const size_t smem = (size_t)n_choices * (nbins_a + nbins_b) * (sizeof(unsigned int) + 1);
-    SSM_REQUIRE(n_sets < (int64_t)1 << 28, "too many sets for one launch");
     cudaStream_t st = (cudaStream_t)stream;
     if (n_choices <= 2) return launch_per_set(k_set_summary<2>, a, n_sets, smem, st);
     if (n_choices <= 4) return launch_per_set(k_set_summary<4>, a, n_sets, smem, st);
@@ -1144,7 +1144,6 @@ int ssm_kde_fit(const float *rts, const int32_t *choices, int64_t n_sets,
     KdeFit a{rts, choices, n_sets, sample_offsets, choice_values, n_choices, displace,
              displace ? displaced_logs : nullptr, count_all, n_valid, point_offsets, points,
              bandwidth, log_norm, proportion};
-    SSM_REQUIRE(n_sets < (int64_t)1 << 28, "too many sets for one launch");
     if (n_choices <= 2) return kde_fit<2>(a, st);
     if (n_choices <= 4) return kde_fit<4>(a, st);
     return kde_fit<KDE_MAX_CHOICES>(a, st);
