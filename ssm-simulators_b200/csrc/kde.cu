@@ -48,12 +48,6 @@ struct KdeFit {
     double *prop;        // [G] choice proportion
 };
 
-__device__ __forceinline__ int choice_index(int32_t ch, const int32_t *cvals, int nc) {
-    for (int c = 0; c < nc; ++c)
-        if (__ldg(cvals + c) == ch) return c;
-    return -1;
-}
-
 // The choice values in registers; NC is the compiled capacity (2, 4 or 16),
 // nc the number in use.
 template <int NC> struct ChoiceSet {
@@ -691,7 +685,6 @@ __global__ void __launch_bounds__(KDE_THREADS, 7) k_kde_eval(const KdeEval a) {
             // this CTA computes the tiles whose first cost index is in [i0, i1)
             const int64_t t0 = (i0 > ubeg) ? (i0 - ubeg + R) / (R + 1) : 0;
             const int64_t t1 = (i1 < uend) ? min((i1 - ubeg + R) / (R + 1), tiles) : tiles;
-            if (t0 >= tiles) continue;
             if (t0 >= t1) continue;
             if (i0 > ubeg && threadIdx.x == 0) a.link[c] = (t1 == tiles) ? SPLIT_LAST : SPLIT_PART;
             const int64_t q0 = qa + 32 * rows.r0;

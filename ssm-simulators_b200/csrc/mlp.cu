@@ -364,11 +364,9 @@ __device__ __forceinline__ void epi_dtanh(uint32_t ta, const uint8_t *H, uint8_t
 }
 
 // same, with h taken from the packed bf16 stash in TMEM
-template <int SPLIT>
-__device__ __forceinline__ void epi_dtanh_stash(uint32_t ta, uint32_t ts, uint8_t *dst, int r, int half) {
-    const int end = last_chunk<SPLIT>(half, N1 / 16);
+__device__ __forceinline__ void epi_dtanh_stash(uint32_t ta, uint32_t ts, uint8_t *dst, int r) {
 #pragma unroll 1
-    for (int c = first_chunk<SPLIT>(half, N1 / 16); c < end; ++c) {
+    for (int c = 0; c < N1 / 16; ++c) {
         float v[16];
         tmem_ld16(ta + 16 * c, v);
         uint32_t hh[8];
@@ -476,6 +474,7 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
       float *__restrict__ out, float *__restrict__ dx, int dx_stride, int loss_kind, float inv_batch,
       float *__restrict__ part, float *__restrict__ part_loss, int *__restrict__ status) {
     constexpr int NWG = Cfg<MODE>::NWG, SPLIT = Cfg<MODE>::SPLIT, TEAM = 128 * SPLIT;
+    static_assert(SPLIT == (MODE == TRAIN ? 2 : 1), "inference has one warpgroup to a tile, training two");
     extern __shared__ __align__(1024) uint8_t sm[];
     const int tid = threadIdx.x, wg = tid / TEAM, half = (tid >> 7) % SPLIT, r = tid & 127, warp = tid >> 5;
     const bool lead = tid % TEAM == 0;  // issues the tile's MMAs
@@ -555,7 +554,7 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                 bar_sync(bid, TEAM);
             }
             const int64_t next = row + stride * 128;
-            const bool more = MODE != TRAIN && half == 0 && tile + stride < n_tiles;
+            const bool more = MODE != TRAIN && tile + stride < n_tiles;
             if (more) load_x(x, x_stride, rt, choice, next < n ? next : 0, xv);
 
             if (MODE != TRAIN) {
@@ -575,7 +574,7 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                 }
                 late |= !mbar_wait(mbar, phase); phase ^= 1;
                 tc_after();
-                epi_hidden<N1, H1, ONES1, MODE == FWD_DX, SPLIT>(tw, B0, r, tstash, half);
+                epi_hidden<N1, H1, ONES1, MODE == FWD_DX, 1>(tw, B0, r, tstash, 0);
                 if (MODE == FWD_DX) tmem_wait_st();
                 tc_before();
                 fence_async_smem();
@@ -589,7 +588,7 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                 if (more) stage_x(X, r, xv, next < n, nm);  // layer 1's MMA has read X
                 late |= !mbar_wait(mbar, phase); phase ^= 1;
                 tc_after();
-                epi_hidden<N2, H2, ONES1, false, SPLIT>(tw, Hb, r, 0, half);
+                epi_hidden<N2, H2, ONES1, false, 1>(tw, Hb, r, 0, 0);
                 tc_before();
                 fence_async_smem();
                 bar_sync(bid, TEAM);
@@ -616,7 +615,7 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                     }
                     late |= !mbar_wait(mbar, phase); phase ^= 1;
                     tc_after();
-                    epi_dtanh<N2, N2, SPLIT>(tw, B1, B1, r, half);   // G2 over h2, in place
+                    epi_dtanh<N2, N2, 1>(tw, B1, B1, r, 0);   // G2 over h2, in place
                     tc_before();
                     fence_async_smem();
                     bar_sync(bid, TEAM);
@@ -628,7 +627,7 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                     }
                     late |= !mbar_wait(mbar, phase); phase ^= 1;
                     tc_after();
-                    epi_dtanh_stash<SPLIT>(tw, tstash, B0, r, half);  // G1 over h1 (stash) -> B0
+                    epi_dtanh_stash(tw, tstash, B0, r);  // G1 over h1 (stash) -> B0
                     tc_before();
                     fence_async_smem();
                     bar_sync(bid, TEAM);
@@ -642,7 +641,7 @@ k_mlp(const uint8_t *__restrict__ image, const float *__restrict__ x, int64_t n,
                     tc_after();
                     float v[16];
                     tmem_ld16(tw, v);
-                    if (valid && half == 0) {
+                    if (valid) {
                         float *d = dx + row * (int64_t)dx_stride;
 #pragma unroll
                         for (int j = 0; j < DIN; ++j) d[j] = v[j] * nm.s[j];
