@@ -79,9 +79,14 @@ typedef struct ssm_launch {
      * With more than one the lanes of a group draw a walk's increments in
      * parallel and share its tests: results are bit-identical to one, and a
      * launch with fewer trajectories than lanes ends sooner.  The library takes
-     * the value as a statement of how short of trajectories the launch is: 8
-     * becomes 16 or 32 when the GPU holds all its walks that way, and 2 and 4
-     * become one lane with the launch's last trajectories on several. */
+     * the value as a statement of how short of trajectories the launch is:
+     *   8  takes 32 lanes up to 24 trajectories per SM and 16 up to 96 (counts
+     *      known to the host: not in the ragged layout), else 8;
+     *   4  takes 8 lanes up to 576 trajectories per SM (not in the ragged layout)
+     *      or if the workspace has no room for handing trajectories over, else as 1;
+     *   2  as 1;
+     *   1  one lane per trajectory; with that room (ssm_ddm_workspace_bytes) a
+     *      launch's last trajectories are handed to groups of eight lanes. */
     int lanes_per_walk;
 } ssm_launch;
 
@@ -100,9 +105,9 @@ int ssm_check_status(const void *workspace, void *stream);
  * lane per walk leaves to several lanes at its end (7.3 MB on 148 SMs; a smaller
  * workspace is accepted, and the launch then ends on one lane per walk). */
 size_t ssm_ddm_workspace_bytes(int64_t n_trials);
-/* Lanes per walk (ssm_launch.lanes_per_walk) the library picks for a
- * single-accumulator launch of n_walks trajectories on the current device
- * when the option is 0 and the layout is not ragged; callers of the ragged
+/* The value of ssm_launch.lanes_per_walk that 0 stands for in a single-accumulator
+ * launch of n_walks trajectories on the current device when the layout is not
+ * ragged (see there for the lanes that each value takes); callers of the ragged
  * layout, which know their total, pass it explicitly.  No reference
  * counterpart: a launch-shape choice of this library. */
 int ssm_auto_lanes_per_walk(int64_t n_walks);

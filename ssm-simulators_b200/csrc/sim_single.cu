@@ -28,9 +28,9 @@
 //    transform, 16-step blocks).
 //  * A launch lasts as long as its longest walk.  When the queue is empty and a
 //    warp has at most LEAVE_MAX walks left, it hands them (LeftWalk) to k_wide
-//    (sim_wide.cu), which gives a walk 8 to 32 lanes; a launch with fewer walks
-//    than the grid has lanes goes there as a whole (ssm_launch.lanes_per_walk).
-//    Outputs are bit-identical to one lane per walk.
+//    (sim_wide.cu), which gives each of them eight lanes; a launch with fewer walks
+//    than the grid has lanes may go there as a whole, on 8, 16 or 32 lanes a walk
+//    (effective_lanes).  Outputs are bit-identical to one lane per walk.
 //  * Boundaries are evaluated in registers (constant / linear collapse /
 //    Weibull) or read from a caller-evaluated table for arbitrary shapes.
 //  * Noise injection replaces the generator by caller rows and switches every
@@ -457,9 +457,6 @@ __global__ void __launch_bounds__(256, 3) k_single(const __grid_constant__ Singl
                 n_next = (uint32_t)(q_next - sp.lo);
             }
         }
-        // (The exit test below stays outside the branch above: with the break inside
-        // it, one of the noise-injection kernels took the claim's shuffled base from
-        // the register of `need` -- found on bounded, index-checked copies.)
         // The queue is empty and few of the warp's walks still run: a walk here
         // takes the time of a whole warp's steps, a walk with eight lanes of its
         // own a tenth of it, so they are left to the lanes-per-walk kernel.
@@ -553,9 +550,10 @@ __global__ void k_record(const __grid_constant__ SingleParams p) {
 }
 
 // ------------------------------------------------------------------ host side
-// Lanes per walk chosen when the caller leaves it at 0: the wide modes pay
-// where a launch holds about as many trajectories as the grid has lanes
-// (the walks' latency sets the time) and cost throughput beyond.
+// What the caller's 0 stands for, by how short of walks the launch is: several
+// lanes per walk pay where it holds fewer than the grid has lanes (the walks'
+// latency sets the time) and cost throughput beyond.  effective_lanes turns the
+// class into lanes.
 int auto_lanes_per_walk(int64_t n_walks) {
     if (n_walks <= 0) return 1;
     const double per_lane = (double)n_walks / ((double)sm_count() * 768.0);  // 24 resident warps per SM
@@ -565,10 +563,12 @@ int auto_lanes_per_walk(int64_t n_walks) {
     return 1;
 }
 
-// The lanes a launch really takes.  Asked for 8, a launch of known size takes wider
-// groups as long as the GPU holds them; asked for 2 or 4 it runs one lane per
-// walk and hands its last walks over (left: it has the room for them), which has
-// overtaken both.  Plain DDM, one parameter set, us for 1 / 4 / 8 / 16 / 32 lanes
+// The lanes a launch really takes.  Asked for 8, a launch of known size takes 32 or
+// 16 as long as the GPU holds all its walks that way.  Asked for 2, it runs one lane
+// per walk and hands its last walks over if it has the room for them (left).
+// Asked for 4, it does so from 24 walks per resident warp on (85 248 on 148 SMs), where
+// both cost the same, and in the ragged layout, whose total the host does not know
+// here; below, and without that room, it takes 8 lanes.  Plain DDM, one parameter set, us for 1 / 4 / 8 / 16 / 32 lanes
 // (one lane without and with handing over): 1 000 walks 266, 160 / 120 / 78 / 57 /
 // 47; 10 000 385, 215 / 175 / 120 / 92 / 106; 30 000 407, 256 / 219 / 161 / 170 /
 // 243; 100 000 613, 353 / 360 / 351 / 445 / 721; 300 000 778, 549 / 749 / 904.

@@ -415,7 +415,9 @@ int launch(const SingleParams &p, const ssm_launch *opt, cudaStream_t st) {
     return SSM_OK;
 }
 
-// The left walks: a tenth of the lanes' number at most, eight lanes each.
+// The left walks, eight lanes each: at most LEAVE_MAX of each warp's 32, which is
+// half of k_single's lanes and six times the groups of this grid; groups that are
+// done take the next ones from the queue.
 template <int MODEL, int BOUND>
 int finish(const SingleParams &p, cudaStream_t st) {
     auto kern = k_wide<MODEL, BOUND, 8>;

@@ -156,10 +156,15 @@ def lanes_per_walk_for(expected_time, walk_cap, n_samples, delta_t: float, lanes
     over the resident lanes (24 warps on every SM); the longest walk is taken
     as max_k min(cap_k, 8 E[T_k]) / dt, since walk durations have an
     exponential tail (the longest of 1e5 plain-DDM walks with mean 1.4 s took
-    11.6 s).  The thresholds on their ratio come from one B200: plain DDM
-    with 1e3 to 3e6 trajectories and angle batches of 16 to 1024 sets of
-    about 1e4 (ratio <= 0.1: 8 lanes, <= 0.35: 4, <= 1: 2, else 1).  ``lanes``
-    defaults to the current device's resident lanes."""
+    11.6 s).  Ratios up to 0.1 give 8, up to 0.35 4, up to 1 2, else 1.  In a ragged
+    launch 8 runs eight lanes to every walk; 4, 2 and 1 all run one, with the
+    launch's last walks on eight (``ssm_launch.lanes_per_walk``).  So 0.1 is the line
+    that counts, drawn when a launch ended on one lane per walk.  Against one lane
+    with hand-over, us for 1 / 8: plain DDM, one set of 1e3, 3e4 and 1e5 walks (ratio
+    0.00, 0.03, 0.11) 172 / 117, 150 / 136, 261 / 320; 16 sets of 1e4, plain DDM (0.09)
+    642 / 544, Weibull (0.14) 771 / 582, full_ddm (0.07) 500 / 518; 8, 16 and 32 angle
+    sets of 1e4 (0.14, 0.10, 0.09) 273 / 263, 259 / 370, 414 / 605.  ``lanes`` defaults to
+    the current device's resident lanes."""
     e = np.asarray(expected_time, np.float64).reshape(-1)
     ns = np.asarray(n_samples, np.float64).reshape(-1)
     if e.size == 0 or ns.sum() <= 0:
