@@ -258,12 +258,12 @@ class ClockSampler:
 
 
 # ------------------------------------------------------------------ GPU side
-# DRAM bytes (read + write) of one k_single launch on the 4096-theta workload,
-# from one ncu capture of that launch (dram__bytes_read.sum 10,086,144 +
-# dram__bytes_write.sum 287,236,864).
-# The algorithmic output is 8 B per trajectory (338 MB); part of it is still in
-# L2 when the kernel ends, so the measured writes sit slightly below it.
-K_SINGLE_TRAFFIC_BYTES = 10_086_144 + 287_236_864
+# DRAM bytes (read + write) of one launch on the 4096-theta workload, from one ncu
+# capture of its three kernels: k_single 11,435,008 + 288,636,672, k_wide (the
+# last walks) 1,872,896 + 12,288, k_finish 169,511,936 + 105,269,760.
+# The algorithmic output is 8 B per trajectory (338 MB); k_finish reads the rts
+# and writes them again (2 x 169 MB, part of it still in L2 when it ends).
+K_SINGLE_TRAFFIC_BYTES = 11_435_008 + 288_636_672 + 1_872_896 + 12_288 + 169_511_936 + 105_269_760
 
 
 def hbm_peak() -> tuple[float, str]:
