@@ -18,6 +18,7 @@ Two ways to drive it:
 from __future__ import annotations
 
 import ctypes as C
+import os
 import subprocess
 from pathlib import Path
 
@@ -40,11 +41,20 @@ class _Noise(C.Structure):
 
 
 def build(force: bool = False) -> Path:
-    """Compile the C restatement (gcc, no fast-math, no FP contraction)."""
+    """Compile the C restatement (gcc, no fast-math, no FP contraction).
+
+    Into a file of this process's own, which then takes the library's place whole:
+    worker processes that find none build it side by side, and none may load
+    another's half-written file."""
     LIB.parent.mkdir(parents=True, exist_ok=True)
     if force or not LIB.exists() or LIB.stat().st_mtime < SRC.stat().st_mtime:
-        subprocess.check_call(["gcc", "-O2", "-ffp-contract=off", "-fno-fast-math", "-fPIC",
-                               "-shared", str(SRC), "-o", str(LIB), "-lm"])
+        tmp = LIB.with_name(f"{LIB.name}.{os.getpid()}")
+        try:
+            subprocess.check_call(["gcc", "-O2", "-ffp-contract=off", "-fno-fast-math", "-fPIC",
+                                   "-shared", str(SRC), "-o", str(tmp), "-lm"])
+            os.replace(tmp, LIB)
+        finally:
+            tmp.unlink(missing_ok=True)
     return LIB
 
 
